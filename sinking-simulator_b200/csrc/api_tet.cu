@@ -83,6 +83,8 @@ TetParams make_params(const femstep_tet* s, const femstep_tet_params& p) {
         // plasticity::Material::shearModulus / bulkModulus (plasticity.hpp:226-227)
         q.mu = E / (2.0 * (1.0 + nu));
         q.bulk = E / (3.0 * (1.0 - 2.0 * nu));
+        q.inv_2mu = 1.0 / (2.0 * q.mu);
+        q.inv_3bulk = 1.0 / (3.0 * q.bulk);
     }
     q.yield = p.yield_strength;
     q.hardening = p.hardening_modulus;
@@ -117,7 +119,7 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
     s->mode = mode;
     s->nodes = N;
     s->tets = T;
-    s->eblocks = fs::blocks_for((long long)T, fs::kBlock);
+    s->eblocks = fs::blocks_for((long long)T, mode == FEMSTEP_TET_J2_F64 ? fs::kTet64Block : fs::kBlock);
     s->nblocks = fs::blocks_for((long long)N, fs::kBlock);
     int rc = check(s, cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "stream");
     if (rc == FEMSTEP_OK) rc = check(s, cudaEventCreate(&s->ev0), "event");
@@ -285,7 +287,7 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
     s->mode = mode;
     s->nodes = N;
     s->tets = T;
-    s->eblocks = fs::blocks_for((long long)T, fs::kBlock);
+    s->eblocks = fs::blocks_for((long long)T, mode == FEMSTEP_TET_J2_F64 ? fs::kTet64Block : fs::kBlock);
     s->nblocks = fs::blocks_for((long long)N, fs::kBlock);
     int rc = check(s, cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "stream");
     if (rc == FEMSTEP_OK) rc = check(s, cudaEventCreate(&s->ev0), "event");
@@ -593,10 +595,11 @@ int femstep_tet_critical_dt(femstep_tet* s, double youngs, double poisson, doubl
         inv = tmp;
     }
     double* block_max = nullptr;
-    rc = check(s, fs::device_alloc((void**)&block_max, sizeof(double) * s->eblocks), "alloc");
+    const int blocks = fs::blocks_for((long long)T, fs::kBlock);
+    rc = check(s, fs::device_alloc((void**)&block_max, sizeof(double) * blocks), "alloc");
     if (!rc) {
-        fs::launch_tet_omega2((long long)T, inv, youngs, poisson, density, block_max, s->eblocks, s->stream);
-        fs::launch_reduce_max(block_max, s->eblocks, s->d_out + 7, s->stream);
+        fs::launch_tet_omega2((long long)T, inv, youngs, poisson, density, block_max, blocks, s->stream);
+        fs::launch_reduce_max(block_max, blocks, s->d_out + 7, s->stream);
         double w2 = 0.0;
         rc = check(s, cudaMemcpyAsync(&w2, s->d_out + 7, sizeof(double), cudaMemcpyDeviceToHost, s->stream), "readback");
         if (!rc) rc = check(s, cudaStreamSynchronize(s->stream), "critical dt");

@@ -71,6 +71,7 @@ struct TetDevice {
 
 struct TetParams {
     double lambda, mu, bulk;      // Lame constants and bulk modulus
+    double inv_2mu, inv_3bulk;    // 1 / (2 mu), 1 / (3 bulk): the energy account
     double yield, hardening;      // J2 linear isotropic hardening
     double dt, gravity, damping;
     int ramp;
@@ -78,6 +79,7 @@ struct TetParams {
 
 // Launchers.  `stream` is the caller's stream; every launch is asynchronous.
 // `parts`: kElementPart | kNodePart (a whole step), or one of them alone (profiling).
+constexpr int kTet64Block = 128;  // threads per block of the FP64 element kernel
 constexpr int kElementPart = 1, kNodePart = 2, kWholeStep = 3;
 void launch_ref32_step(const TetDevice<float>& d, const TetParams& p, cudaStream_t stream,
                        int parts = kWholeStep);

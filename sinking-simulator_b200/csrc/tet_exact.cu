@@ -37,22 +37,156 @@ __device__ __forceinline__ M3<float> polar_fixed4(const M3<float>& f) {
     return r;
 }
 
-__device__ __forceinline__ M3<double> polar_converged(const M3<double>& f) {
-    M3<double> r = f;
-#pragma unroll 1
-    for (int it = 0; it < 64; ++it) {
-        if (det3(r) == 0.0) return r;
-        const M3<double> rit = transpose(inverse(r, 1e-300));
-        double worst = 0.0;
+// One step of it; true once the iteration ends there (converged, or singular).
+__device__ __forceinline__ bool polar_step(M3<double>& r) {
+    if (det3(r) == 0.0) return true;
+    const M3<double> rit = transpose(inverse(r, 1e-300));
+    double worst = 0.0;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const double next = 0.5 * (r.m[k] + rit.m[k]);
-            const double d = fabs(next - r.m[k]);
-            worst = worst > d ? worst : d;
-            r.m[k] = next;
-        }
-        if (worst < 1e-16) return r;
+    for (int k = 0; k < 9; ++k) {
+        const double next = 0.5 * (r.m[k] + rit.m[k]);
+        const double d = fabs(next - r.m[k]);
+        worst = worst > d ? worst : d;
+        r.m[k] = next;
     }
+    return worst < 1e-16;
+}
+
+// The same step where det x is 1 to within 2^-30, as it is from the third step on for
+// any moderate strain; returns det x, for the caller to check.  A step is a chain of
+// dependent FP64 operations, and there it can be shortened without changing a bit:
+//   * 1 / det is 2 - det rounded up.  With det = 1 + m 2^-52 (0 < m <= 2^22), 1 / det is
+//     2 - det, which is a double, plus at most m^2 2^-104, far under half its ulp; with
+//     det = 1 - m 2^-53 it is 1 + m 2^-53 plus a little over m^2 2^-106, so it rounds to
+//     2 - det where that is a double (m even) and up from the midpoint where it is not.
+//   * 0.5 (r + c / det) is fma(0.5, r, c (0.5 / det)): halving is exact (the cofactors of
+//     positions' differences are zero or far above the subnormals).
+// Eight operations deep instead of the divide and ten.
+__device__ __forceinline__ double polar_near(const M3<double>& r, M3<double>& y) {
+    const double c00 = r(1, 1) * r(2, 2) - r(1, 2) * r(2, 1), c01 = r(1, 0) * r(2, 2) - r(1, 2) * r(2, 0),
+                 c02 = r(1, 0) * r(2, 1) - r(1, 1) * r(2, 0);
+    const double det = r(0, 0) * c00 - r(0, 1) * c01 + r(0, 2) * c02;
+    // the transposed inverse's numerators, in inverse()'s own order of terms
+    const double c[9] = {c00,
+                         r(0, 2) * r(2, 1) - r(0, 1) * r(2, 2),
+                         r(0, 1) * r(1, 2) - r(0, 2) * r(1, 1),
+                         r(1, 2) * r(2, 0) - r(1, 0) * r(2, 2),
+                         r(0, 0) * r(2, 2) - r(0, 2) * r(2, 0),
+                         r(0, 2) * r(1, 0) - r(0, 0) * r(1, 2),
+                         c02,
+                         r(0, 1) * r(2, 0) - r(0, 0) * r(2, 1),
+                         r(0, 0) * r(1, 1) - r(0, 1) * r(1, 0)};
+    const double half = __fma_ru(-0.5, det, 1.0);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) y.m[k] = __fma_rn(0.5, r.m[k], c[k] * half);
+    return det;
+}
+
+// Negative where |y_k - x_k| is under 1e-16 (all finite) for every k in `from`, `from` +
+// `by`, ...: the signs of the bit patterns' differences, ANDed.
+template <int FROM, int BY>
+__device__ __forceinline__ int polar_still(const M3<double>& x, const M3<double>& y) {
+    int all = -1;
+#pragma unroll
+    for (int k = FROM; k < 9; k += BY) {
+        const long long bits = __double_as_longlong(fabs(y.m[k] - x.m[k])) - __double_as_longlong(1e-16);
+        all &= (int)(bits >> 32);
+    }
+    return all;
+}
+
+// Two steps; true once the iteration has ended (x is then its result).  Almost every
+// step that goes on shows it on the diagonal alone (an ulp there is more than 1e-16), so
+// the three diagonal entries are tested first, and the two steps' tests are decided
+// together beside the second step's arithmetic.
+__device__ __forceinline__ bool polar_pair(M3<double>& x) {
+    M3<double> y, z;
+    const double d0 = polar_near(x, y), d1 = polar_near(y, z);
+    const bool near = fabs(d0 - 1.0) <= 0x1p-30 && fabs(d1 - 1.0) <= 0x1p-30;
+    if (near && (polar_still<0, 4>(x, y) | polar_still<0, 4>(y, z)) >= 0) {
+        x = z;
+        return false;
+    }
+    if (near) {
+        if (polar_still<0, 1>(x, y) < 0) {
+            x = y;
+            return true;
+        }
+        const bool end = polar_still<0, 1>(y, z) < 0;
+        x = z;
+        return end;
+    }
+    return polar_step(x) || polar_step(x);
+}
+
+// The iteration for a block's tets together.  Two thirds of moving tets end within six
+// steps; the others never meet the test, because the last bits go round (a period of 2
+// or 3) or drift, and take all 64 steps.  One tet a lane, nearly every warp would run 64
+// steps for a third of its lanes.  So the block packs the unfinished tets into its first
+// warps after six steps and again after sixteen, and there leaves out those that are
+// where they were six steps before: 48 more steps bring them back to the same bits.
+// Every tet ends with the bits of its own 64-step loop.  F and the tet's rows wait in
+// shared memory too, so that a block holds few registers while most of its warps wait
+// for the packed ones: five blocks an SM (96 registers) where four measured 128 us a
+// step, on the 480,000-tet beam in motion, and five 113 us.  One tet a lane with the
+// divide in every step took 218 us there, and 34.4 us a step (now 22.6 us) on the
+// 3,840-tet cantilever, where the 64 steps of one warp are the pass: 207 cycles each,
+// 122 of them issuing its FP64 operations at two cycles each.
+struct PolarPark {
+    double rows[17][kTet64Block];  // Dm^-1, volume, plastic state: copied in while F is formed
+    double f[9][kTet64Block];
+    double r[9][kTet64Block];
+    uint16_t list[2][kTet64Block];
+    int count[2];
+};
+
+__device__ __forceinline__ M3<double> polar_block(M3<double> r, bool live, PolarPark& park) {
+    constexpr int kFirst = 6, kSnapshot = 10, kSecond = 16, kLast = 64;
+    static_assert((kLast - kSecond) % (kSecond - kSnapshot) == 0, "whole periods remain");
+    static_assert(kFirst % 2 == 0 && kSnapshot % 2 == 0 && kSecond % 2 == 0 && kLast % 2 == 0, "steps go in pairs");
+    const int tid = threadIdx.x;
+    if (tid < 2) park.count[tid] = 0;
+    __syncthreads();
+    bool done = !live || polar_step(r) || polar_step(r);
+#pragma unroll 1
+    for (int it = 2; it < kFirst && !done; it += 2) done = polar_pair(r);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) park.r[k][tid] = r.m[k];
+    if (!done) park.list[0][atomicAdd(&park.count[0], 1)] = (uint16_t)tid;
+#pragma unroll 1
+    for (int round = 0; round < 2; ++round) {
+        __syncthreads();
+        const int n = park.count[round];
+        if (n == 0) break;  // the same for the whole block
+        if (tid < n) {
+            const int at = park.list[round][tid];
+            M3<double> x;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) x.m[k] = park.r[k][at];
+            bool end = false;
+            const int last = round ? kLast : kSecond;
+#pragma unroll 1
+            for (int it = round ? kSecond : kFirst; it < last && !end; it += 2) {
+                if (it == kSnapshot) {
+#pragma unroll
+                    for (int k = 0; k < 9; ++k) park.r[k][at] = x.m[k];
+                }
+                end = polar_pair(x);
+            }
+            if (!end && !round) {
+                bool same = true;
+#pragma unroll
+                for (int k = 0; k < 9; ++k)
+                    same = same && __double_as_longlong(x.m[k]) == __double_as_longlong(park.r[k][at]);
+                if (!same) park.list[1][atomicAdd(&park.count[1], 1)] = (uint16_t)at;
+            }
+#pragma unroll
+            for (int k = 0; k < 9; ++k) park.r[k][at] = x.m[k];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 9; ++k) r.m[k] = park.r[k][tid];
     return r;
 }
 
@@ -154,11 +288,12 @@ __global__ void __launch_bounds__(kBlock) ref32_nodes(TetDevice<float> d, float 
 // arithmetic order is the CPU's, term for term.
 struct J2Out {
     double dissipation;
+    bool yielded;
 };
 
 __device__ __forceinline__ J2Out j2_return_f64(const double strain[6], double ps[7], double mu, double kappa,
                                                double yield, double hardening, double stress[6]) {
-    J2Out out{0.0};
+    J2Out out{0.0, false};
     const double root23 = sqrt(2.0 / 3.0);
     double elastic[6];
 #pragma unroll
@@ -188,6 +323,7 @@ __device__ __forceinline__ J2Out j2_return_f64(const double strain[6], double ps
         }
         return out;
     }
+    out.yielded = true;
     const double linear_part = 2.0 * mu + (2.0 / 3.0) * 0.0;
     double lo = 0.0, hi = excess / linear_part;
     double gamma = hi;
@@ -234,8 +370,9 @@ __device__ __forceinline__ J2Out j2_return_f64(const double strain[6], double ps
     return out;
 }
 
-__global__ void __launch_bounds__(kBlock) f64_forces(TetDevice<double> d, TetParams p) {
-    __shared__ double scratch[32];
+__global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d, TetParams p) {
+    __shared__ double scratch[64];
+    __shared__ PolarPark park;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const long long s = d.counter[0];
@@ -243,19 +380,36 @@ __global__ void __launch_bounds__(kBlock) f64_forces(TetDevice<double> d, TetPar
         d.counter[0] = s + 1;
     }
     double diss = 0.0, energy = 0.0;
-    if (t < d.tets) {
+    const bool live = t < d.tets;
+    M3<double> f;
+    if (live) {
         const uint4 idx = d.index[t];
         const unsigned nid[4] = {idx.x, idx.y, idx.z, idx.w};
         const double* x = d.position;
         M3<double> ds, dm_inv;
 #pragma unroll
+        for (int k = 0; k < 9; ++k) cp_async8(&park.rows[k][threadIdx.x], d.rest_inv + (size_t)k * d.tets + t);
+        cp_async_commit();
+        cp_async8(&park.rows[9][threadIdx.x], d.rest_vol + t);
+#pragma unroll
+        for (int i = 0; i < 7; ++i) cp_async8(&park.rows[10 + i][threadIdx.x], d.plastic + (size_t)i * d.tets + t);
+        cp_async_commit();
+#pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
             for (int a = 0; a < 3; ++a) ds(a, c) = x[(size_t)nid[c + 1] * 3 + a] - x[(size_t)nid[0] * 3 + a];
+        cp_async_wait_one();  // a thread reads back only what it copied: no barrier
 #pragma unroll
-        for (int k = 0; k < 9; ++k) dm_inv.m[k] = d.rest_inv[(size_t)k * d.tets + t];
-        const M3<double> f = mul(ds, dm_inv);
-        const M3<double> r = polar_converged(f);
+        for (int k = 0; k < 9; ++k) dm_inv.m[k] = park.rows[k][threadIdx.x];
+        f = mul(ds, dm_inv);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) park.f[k][threadIdx.x] = f.m[k];
+    }
+    const M3<double> r = polar_block(f, live, park);
+    if (live) {
+        cp_async_wait_all();
+#pragma unroll
+        for (int k = 0; k < 9; ++k) f.m[k] = park.f[k][threadIdx.x];
         const M3<double> sm = mul(transpose(r), f);
         double strain[6];
         strain[0] = 0.5 * (sm(0, 0) + sm(0, 0)) - 1.0;
@@ -266,21 +420,24 @@ __global__ void __launch_bounds__(kBlock) f64_forces(TetDevice<double> d, TetPar
         strain[5] = 2.0 * (0.5 * (sm(2, 0) + sm(0, 2)));
         double ps[7];
 #pragma unroll
-        for (int i = 0; i < 7; ++i) ps[i] = d.plastic[(size_t)i * d.tets + t];
+        for (int i = 0; i < 7; ++i) ps[i] = park.rows[10 + i][threadIdx.x];
         double sv[6];
         const J2Out j = j2_return_f64(strain, ps, p.mu, p.bulk, p.yield, p.hardening, sv);
+        if (j.yielded) {
 #pragma unroll
-        for (int i = 0; i < 7; ++i) d.plastic[(size_t)i * d.tets + t] = ps[i];
-        const double vol = d.rest_vol[t];
+            for (int i = 0; i < 7; ++i) d.plastic[(size_t)i * d.tets + t] = ps[i];
+        }
+        const double vol = park.rows[9][threadIdx.x];
         diss = vol * j.dissipation;
-        const double pressure = (sv[0] + sv[1] + sv[2]) / 3.0;
-        double density = 0.0;
+        // 1/2 sigma : C^-1 : sigma from the deviator and the trace, by the reciprocals
+        const double tr = sv[0] + sv[1] + sv[2], pressure = tr * (1.0 / 3.0);
+        const double e0 = sv[0] - pressure, e1 = sv[1] - pressure, e2 = sv[2] - pressure;
+        const double dev = e0 * e0 + e1 * e1 + e2 * e2 + 2.0 * (sv[3] * sv[3] + sv[4] * sv[4] + sv[5] * sv[5]);
+        energy = 0.5 * vol * (dev * p.inv_2mu + pressure * tr * p.inv_3bulk);
+
+        M3<double> dm_inv;
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
-            density += 0.5 * sv[i] * ((sv[i] - pressure) / (2.0 * p.mu) + pressure / (3.0 * p.bulk));
-#pragma unroll
-        for (int i = 3; i < 6; ++i) density += 0.5 * sv[i] * (sv[i] / p.mu);
-        energy = vol * density;
+        for (int k = 0; k < 9; ++k) dm_inv.m[k] = park.rows[k][threadIdx.x];
 
         M3<double> stress;
         stress(0, 0) = sv[0];
@@ -308,11 +465,10 @@ __global__ void __launch_bounds__(kBlock) f64_forces(TetDevice<double> d, TetPar
 #pragma unroll
         for (int a = 0; a < 3; ++a) out0[a] = f0[a];
     }
-    const double bd = block_sum(diss, scratch);
-    const double be = block_sum(energy, scratch);
+    block_sum2(diss, energy, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
-        d.e_diss[blockIdx.x] += bd;
-        d.e_strain[blockIdx.x] = be;
+        d.e_diss[blockIdx.x] += diss;
+        d.e_strain[blockIdx.x] = energy;
     }
 }
 
@@ -522,7 +678,7 @@ void launch_ref32_step(const TetDevice<float>& d, const TetParams& p, cudaStream
 }
 
 void launch_f64_step(const TetDevice<double>& d, const TetParams& p, cudaStream_t stream, int parts) {
-    if (parts & kElementPart) f64_forces<<<blocks_for(d.tets, kBlock), kBlock, 0, stream>>>(d, p);
+    if (parts & kElementPart) f64_forces<<<blocks_for(d.tets, kTet64Block), kTet64Block, 0, stream>>>(d, p);
     if (parts & kNodePart) f64_nodes<<<blocks_for(d.nodes, kBlock), kBlock, 0, stream>>>(d, p);
 }
 

@@ -182,3 +182,27 @@ def test_device_set_up_is_the_host_set_up(fem, mode):
     assert np.array_equal(dev.plastic(), host.plastic())
     assert (host.plastic()[:, 6] > 0).any(), "the case must yield"
     assert np.array_equal(dev.energy(), host.energy())
+
+
+@pytest.mark.parametrize("cells", [(7, 3, 1), (16, 4, 1), (43, 1, 1), (13, 5, 2)])
+@pytest.mark.parametrize("pull", [2e4, 2e7])
+def test_f64_at_block_edges_and_large_rotations(fem, port, cells, pull):
+    """The FP64 step packs a block's unfinished polar iterations together: meshes of 126
+    to 780 tets, around one to six blocks' edges and with ragged last ones, from small
+    strains (iterations that cycle or drift in the last bits) to rotations and stretches
+    of order one, bit-identical to the FP64 oracle."""
+    nx, ny, nz = cells
+    pos, idx = fem.box_tet_mesh(0.1 * nx, 0.1 * ny, 0.1 * nz, nx, ny, nz)
+    fixed = (pos[0::3] < 1e-6).astype(np.uint32)
+    tip = pos[0::3] > 0.1 * nx - 1e-6
+    fext = np.zeros(pos.size)
+    fext[2::3][tip] = -pull * ny * nz / tip.sum()
+    ref = O.TetMesh64(port, pos, idx, fixed, fext)
+    dt = 0.5 * port.tet64_critical_dt(C.byref(ref._s), 210e9, 0.3, 7850.0, 0.9)
+    ref.step(O.tet64_params(dt=dt, ramp_steps=100), 400)
+    assert np.isfinite(ref.position).all()
+    g = fem.TetSolver(pos, idx, mode="f64", fixed=fixed, external_force=fext, density=7850.0)
+    g.run(400, dt=dt, ramp_steps=100)
+    p, v = g.readback64()
+    assert np.array_equal(p, ref.position) and np.array_equal(v, ref.velocity)
+    assert np.array_equal(g.plastic().reshape(-1), ref.plastic)
