@@ -120,7 +120,7 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
     s->nodes = N;
     s->tets = T;
     s->eblocks = fs::blocks_for((long long)T, mode == FEMSTEP_TET_J2_F64 ? fs::kTet64Block : fs::kBlock);
-    s->nblocks = fs::blocks_for((long long)N, fs::kBlock);
+    s->nblocks = fs::blocks_for((long long)N, fs::kTetNodeBlock);
     int rc = check(s, cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "stream");
     if (rc == FEMSTEP_OK) rc = check(s, cudaEventCreate(&s->ev0), "event");
     if (rc == FEMSTEP_OK) rc = check(s, cudaEventCreate(&s->ev1), "event");
@@ -134,8 +134,9 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         for (size_t n = 0; n < N; ++n) fixed[n] = m.fixed[n] ? 1 : 0;
     const uint32_t* index = A.upload(m.index, T * 4);
     const float* pos32 = A.upload(m.position, N * 3);
-    uint32_t* offset = A.alloc<uint32_t>(N + 1);
+    uint2* run = A.alloc<uint2>(N);
     uint32_t* slot = A.alloc<uint32_t>(T * 4);
+    long long slots = 0;
     // the FP64 rest state: Dm^-1 (SoA) and volumes per tet, lumped masses per node
     double* inv64 = A.alloc<double>(T * 9);
     double* vol64 = A.alloc<double>(T);
@@ -146,9 +147,10 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         femstep_tet_destroy(s);
         return code;
     }
-    uint32_t* entry = nullptr;
+    uint32_t *entry = nullptr, *offset = nullptr;
     double* quarter = nullptr;
     rc = check(s, fs::device_alloc((void**)&entry, T * 4 * sizeof(uint32_t)), "alloc");
+    if (!rc) rc = check(s, fs::device_alloc((void**)&offset, (N + 1) * sizeof(uint32_t)), "alloc");
     if (!rc) rc = check(s, fs::device_alloc((void**)&quarter, T * sizeof(double)), "alloc");
     if (!rc) rc = check(s, fs::build_csr_device(index, (long long)T * 4, (long long)N, offset, slot, s->stream, entry),
                         "adjacency");
@@ -157,6 +159,8 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         fs::launch_tet_mass64(offset, entry, (long long)N, quarter, mass64, s->stream);
         rc = check(s, cudaGetLastError(), "rest state");
     }
+    if (!rc) rc = check(s, fs::build_runs_device(offset, entry, (long long)T * 4, (long long)N, run, slot, &slots, s->stream),
+                        "slot runs");
 
     auto common = [&](auto& d) {
         d.nodes = (long long)N;
@@ -164,13 +168,17 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         d.index = reinterpret_cast<const uint4*>(index);
         d.slot = reinterpret_cast<const uint4*>(slot);
         d.fixed = A.upload(fixed.data(), N);
-        d.offset = offset;
-        d.counter = A.zeros<long long>(2);
-        d.e_diss = A.zeros<double>(s->eblocks);
-        d.e_strain = A.zeros<double>(s->eblocks);
-        d.n_work = A.zeros<double>(s->nblocks);
-        d.n_kin = A.zeros<double>(s->nblocks);
-        d.n_grav = A.zeros<double>(s->nblocks);
+        d.run = run;
+        d.slot_count = slots;
+        // the step counter, the energy partials and the reductions' output, in one piece
+        double* zero = A.zeros<double>(8 + 2 + 2 * (size_t)s->eblocks + 3 * (size_t)s->nblocks);
+        s->d_out = zero;
+        d.counter = reinterpret_cast<long long*>(zero + 8);
+        d.e_diss = zero + 10;
+        d.e_strain = d.e_diss + s->eblocks;
+        d.n_work = d.e_strain + s->eblocks;
+        d.n_kin = d.n_work + s->nblocks;
+        d.n_grav = d.n_kin + s->nblocks;
     };
     if (!rc && mode == FEMSTEP_TET_J2_F64) {
         TetDevice<double>& d = s->d64;
@@ -178,23 +186,23 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         double* pos = A.alloc<double>(N * 3);
         if (pos) fs::launch_widen(pos32, (long long)N * 3, pos, s->stream);
         d.position = pos;
-        std::vector<double> vel(N * 3, 0.0);
-        if (m.velocity)
-            for (size_t i = 0; i < N * 3; ++i) vel[i] = m.velocity[i];
-        d.velocity = A.upload(vel.data(), N * 3);
+        if (m.velocity) {
+            std::vector<double> vel(m.velocity, m.velocity + N * 3);
+            d.velocity = A.upload(vel.data(), N * 3);
+        } else {
+            d.velocity = A.zeros<double>(N * 3);
+        }
         d.mass = mass64;
         d.rest_inv = inv64;
         d.rest_vol = vol64;
         d.plastic = A.zeros<double>(T * 7);
         if (m.external_force) d.ext = A.upload(m.external_force, N * 3);
-        d.slots = A.zeros<double>(T * 4 * 3 + 2);
+        d.slots = A.alloc<double>((size_t)slots * 3);
     } else if (!rc) {
         TetDevice<float>& d = s->d32;
         common(d);
-        std::vector<float> vel(N * 3, 0.0f);
-        if (m.velocity) std::memcpy(vel.data(), m.velocity, sizeof(float) * N * 3);
-        d.velocity = A.upload(vel.data(), N * 3);
-        d.slots = A.zeros<float>(T * 4 * 4 + 4);  // a padded float4 per corner
+        d.velocity = m.velocity ? A.upload(m.velocity, N * 3) : A.zeros<float>(N * 3);
+        d.slots = A.alloc<float>((size_t)slots * 4);  // a padded float4 per corner
         s->rest.assign(m.position, m.position + N * 3);
         d.rest = pos32;
         d.disp = A.zeros<float>(N * 4);
@@ -219,9 +227,9 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         }
         s->inv64 = inv64;
     }
-    s->d_out = A.zeros<double>(8);
     if (!rc) rc = check(s, cudaStreamSynchronize(s->stream), "set-up");
     fs::device_free(entry);
+    fs::device_free(offset);
     fs::device_free(quarter);
     if (!rc && !A.ok()) {
         const int code = A.status() == cudaErrorMemoryAllocation ? FEMSTEP_ENOMEM : FEMSTEP_ECUDA;
@@ -270,14 +278,16 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
     } else {
         fs::build_csr(N, T, 4, m.index, offset, entry);
     }
-    std::vector<uint32_t> slot(T * 4, 0xffffffffu);
-    for (size_t n = 0; n < N; ++n)
-        for (uint32_t k = offset[n]; k < offset[n + 1]; ++k) {
-            const uint32_t e = entry[k];
-            if (e >= T * 4 || m.index[e] != n || slot[e] != 0xffffffffu)
-                return fail(nullptr, FEMSTEP_EINVAL, "adjacency is not the node-to-corner map of this mesh");
-            slot[e] = k;
-        }
+    {
+        std::vector<bool> seen(T * 4, false);
+        for (size_t n = 0; n < N; ++n)
+            for (uint32_t k = offset[n]; k < offset[n + 1]; ++k) {
+                const uint32_t e = entry[k];
+                if (e >= T * 4 || m.index[e] != n || seen[e])
+                    return fail(nullptr, FEMSTEP_EINVAL, "adjacency is not the node-to-corner map of this mesh");
+                seen[e] = true;
+            }
+    }
     // The mesh is checked before the device, so a bad mesh is reported as such on any
     // machine; a good one on a machine with no GPU is a skip.
     const int dev = fs::device_status();
@@ -288,7 +298,7 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
     s->nodes = N;
     s->tets = T;
     s->eblocks = fs::blocks_for((long long)T, mode == FEMSTEP_TET_J2_F64 ? fs::kTet64Block : fs::kBlock);
-    s->nblocks = fs::blocks_for((long long)N, fs::kBlock);
+    s->nblocks = fs::blocks_for((long long)N, fs::kTetNodeBlock);
     int rc = check(s, cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "stream");
     if (rc == FEMSTEP_OK) rc = check(s, cudaEventCreate(&s->ev0), "event");
     if (rc == FEMSTEP_OK) rc = check(s, cudaEventCreate(&s->ev1), "event");
@@ -304,19 +314,43 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
     std::vector<double> inv64, vol64, mass64;
     if (mode != FEMSTEP_TET_REF32) rest_state64(m, inv64, vol64, mass64);
 
+    uint2* run = A.alloc<uint2>(N);
+    uint32_t* slot = A.alloc<uint32_t>(T * 4);
+    long long slots = 0;
+    {
+        uint32_t *doffset = nullptr, *dentry = nullptr;
+        rc = check(s, fs::device_alloc((void**)&doffset, (N + 1) * sizeof(uint32_t)), "alloc");
+        if (!rc) rc = check(s, fs::device_alloc((void**)&dentry, T * 4 * sizeof(uint32_t)), "alloc");
+        if (!rc) rc = check(s, cudaMemcpy(doffset, offset.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
+        if (!rc) rc = check(s, cudaMemcpy(dentry, entry.data(), T * 4 * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
+        if (!rc && A.ok())
+            rc = check(s, fs::build_runs_device(doffset, dentry, (long long)T * 4, (long long)N, run, slot, &slots, s->stream),
+                       "slot runs");
+        fs::device_free(doffset);
+        fs::device_free(dentry);
+        if (rc) {
+            femstep_tet_destroy(s);
+            return rc;
+        }
+    }
+
     auto common = [&](auto& d) {
         d.nodes = (long long)N;
         d.tets = (long long)T;
         d.index = (const uint4*)A.upload(m.index, T * 4);
-        d.slot = (const uint4*)A.upload(slot.data(), T * 4);
+        d.slot = reinterpret_cast<const uint4*>(slot);
         d.fixed = A.upload(fixed.data(), N);
-        d.offset = A.upload(offset.data(), N + 1);
-        d.counter = A.zeros<long long>(2);
-        d.e_diss = A.zeros<double>(s->eblocks);
-        d.e_strain = A.zeros<double>(s->eblocks);
-        d.n_work = A.zeros<double>(s->nblocks);
-        d.n_kin = A.zeros<double>(s->nblocks);
-        d.n_grav = A.zeros<double>(s->nblocks);
+        d.run = run;
+        d.slot_count = slots;
+        // the step counter, the energy partials and the reductions' output, in one piece
+        double* zero = A.zeros<double>(8 + 2 + 2 * (size_t)s->eblocks + 3 * (size_t)s->nblocks);
+        s->d_out = zero;
+        d.counter = reinterpret_cast<long long*>(zero + 8);
+        d.e_diss = zero + 10;
+        d.e_strain = d.e_diss + s->eblocks;
+        d.n_work = d.e_strain + s->eblocks;
+        d.n_kin = d.n_work + s->nblocks;
+        d.n_grav = d.n_kin + s->nblocks;
     };
 
     if (mode == FEMSTEP_TET_J2_F64) {
@@ -334,16 +368,12 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
         d.rest_vol = A.upload(vol64.data(), T);
         d.plastic = A.zeros<double>(T * 7);
         if (m.external_force) d.ext = A.upload(m.external_force, N * 3);
-        d.slots = A.zeros<double>(T * 4 * 3 + 2);
+        d.slots = A.alloc<double>((size_t)slots * 3);
     } else {
         TetDevice<float>& d = s->d32;
         common(d);
-        std::vector<float> vel(N * 3, 0.0f);
-        if (m.velocity) std::memcpy(vel.data(), m.velocity, sizeof(float) * N * 3);
-        d.velocity = A.upload(vel.data(), N * 3);
-        // REF32: three floats per corner (the reference's layout); J2 modes: a padded
-        // float4 per corner, one 16-byte store each
-        d.slots = A.zeros<float>(mode == FEMSTEP_TET_REF32 ? T * 4 * 3 + 4 : T * 4 * 4 + 4);
+        d.velocity = m.velocity ? A.upload(m.velocity, N * 3) : A.zeros<float>(N * 3);
+        d.slots = A.alloc<float>((size_t)slots * 4);  // a padded float4 per corner, one 16-byte store each
         if (mode == FEMSTEP_TET_REF32) {
             d.position = A.upload(m.position, N * 3);
             d.mass = A.upload(m.mass, N);
@@ -377,7 +407,6 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
         }
     }
     if (mode != FEMSTEP_TET_REF32) s->rest_inv64 = std::move(inv64);
-    s->d_out = A.zeros<double>(8);
     if (!A.ok()) {
         const int code = A.status() == cudaErrorMemoryAllocation ? FEMSTEP_ENOMEM : FEMSTEP_ECUDA;
         fail(s, code, std::string("device upload failed: ") + cudaGetErrorString(A.status()));

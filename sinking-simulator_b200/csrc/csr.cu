@@ -15,6 +15,7 @@
 
 #include "common.cuh"
 #include "shell.hpp"
+#include "tet.hpp"
 
 namespace fs {
 namespace {
@@ -52,12 +53,67 @@ __global__ void csr_slots(const uint32_t* entry, const uint32_t* counted, uint32
         slot[entry[k]] = base + (uint32_t)k;
 }
 
+// The strided layout of the nodes' slot runs (build_runs_device): a warp takes a group of
+// 32 consecutive nodes.
+__device__ __forceinline__ bool run_strided(uint32_t longest, uint32_t sum, bool allow) {
+    return allow && (unsigned long long)longest * 32 <= 2ull * sum;
+}
+
+__global__ void run_spans(const uint32_t* offset, long long nodes, bool allow, uint32_t* span) {
+    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t count = n < nodes ? offset[n + 1] - offset[n] : 0u;
+    const uint32_t longest = __reduce_max_sync(0xffffffffu, count), sum = __reduce_add_sync(0xffffffffu, count);
+    // one more group than there are, so that the scan ends with the total
+    if ((n & 31) == 0 && n < nodes + 32) span[n >> 5] = run_strided(longest, sum, allow) ? 32 * longest : sum;
+}
+
+__global__ void run_fill(const uint32_t* offset, const uint32_t* entry, long long nodes, bool allow,
+                         const uint32_t* base, uint2* run, uint32_t* slot) {
+    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const uint32_t b = n < nodes ? offset[n] : 0u, count = n < nodes ? offset[n + 1] - b : 0u;
+    const uint32_t longest = __reduce_max_sync(0xffffffffu, count), sum = __reduce_add_sync(0xffffffffu, count);
+    const uint32_t first = __shfl_sync(0xffffffffu, b, 0);
+    if (n >= nodes) return;
+    const bool strided = run_strided(longest, sum, allow);
+    const uint32_t start = base[n >> 5] + (strided ? (uint32_t)lane : b - first), step = strided ? 32u : 1u;
+    run[n] = make_uint2(start, count | (strided ? kRunStrided : 0u));
+    for (uint32_t k = 0; k < count; ++k) slot[entry[b + k]] = start + k * step;
+}
+
 __global__ void csr_add_base(uint32_t* offset, long long n, uint32_t base) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         offset[i] += base;
 }
 
 }  // namespace
+
+cudaError_t build_runs_device(const uint32_t* offset, const uint32_t* entry, long long total, long long nodes, uint2* run,
+                              uint32_t* slot, long long* slots, cudaStream_t stream) {
+    const int groups = blocks_for(nodes, 32) + 1;
+    const bool allow = total < (1ll << 30);  // padded runs at most double the slots: 32-bit ids hold them
+    uint32_t* span = nullptr;
+    void* temp = nullptr;
+    size_t temp_bytes = 0;
+    uint32_t count = 0;
+    cudaError_t err = cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, span, span, groups, stream);
+    const size_t scan_at = ((size_t)groups * 2 * sizeof(uint32_t) + 255) & ~size_t(255);
+    if (err == cudaSuccess) err = cudaMallocAsync(&span, scan_at + temp_bytes, stream);
+    if (err == cudaSuccess) {
+        temp = reinterpret_cast<char*>(span) + scan_at;
+        run_spans<<<blocks_for(nodes + 32, 256), 256, 0, stream>>>(offset, nodes, allow, span);
+        err = cub::DeviceScan::ExclusiveSum(temp, temp_bytes, span, span + groups, groups, stream);
+    }
+    if (err == cudaSuccess) {
+        run_fill<<<blocks_for(nodes, 256), 256, 0, stream>>>(offset, entry, nodes, allow, span + groups, run, slot);
+        cudaMemcpyAsync(&count, span + 2 * groups - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
+        err = cudaGetLastError();
+    }
+    if (span) cudaFreeAsync(span, stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+    *slots = count;
+    return err;
+}
 
 cudaError_t build_csr_device(const uint32_t* index, long long total, long long nodes, uint32_t* offset, uint32_t* slot,
                              cudaStream_t stream, uint32_t* entry_out, uint32_t base) {

@@ -22,7 +22,7 @@ __device__ __forceinline__ TetElementRefs element_refs(const PoolDevice& d) {
 }
 
 __device__ __forceinline__ TetNodeRefs node_refs(const PoolDevice& d) {
-    return TetNodeRefs{d.offset, d.slots, d.fixed, d.mass, d.inv_mass, d.ext, d.velocity, d.disp, d.disp_c};
+    return TetNodeRefs{d.slots, d.fixed, d.mass, d.inv_mass, d.ext, d.velocity, d.disp, d.disp_c};
 }
 
 // One element tile at sub-step `sub` of the chunk (all threads of the block call it).
@@ -57,7 +57,8 @@ __device__ __forceinline__ void node_tile(const PoolDevice& d, int tile, int sub
     const long long n = tl.begin + threadIdx.x;
     if (live && n < tl.end) {
         const float lf = (float)ramp_factor(step, m.ramp);
-        tet_node_f32<true, CG>(node_refs(d), n, lf, m.dt, m.gravity, m.damping, work, kin, gwork);
+        const SlotRun run{d.offset[n], d.offset[n + 1] - d.offset[n], 1u};
+        tet_node_f32<true, CG, 0>(node_refs(d), run, n, lf, m.dt, m.gravity, m.damping, work, kin, gwork);
     }
     work += gwork;
     block_sum2(work, kin, scratch);  // valid in thread 0

@@ -231,23 +231,22 @@ __global__ void __launch_bounds__(kBlock) ref32_forces(TetDevice<float> d, float
     const uint4 sl = d.slot[t];
     const unsigned sid[4] = {sl.x, sl.y, sl.z, sl.w};
     float f0[3] = {0.0f, 0.0f, 0.0f};
+    float4* slots = reinterpret_cast<float4*>(d.slots);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        float* out = d.slots + (size_t)sid[c + 1] * 3;
+        float v[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            const float v = scale * h(a, c);
-            out[a] = v;
-            f0[a] -= v;
+            v[a] = scale * h(a, c);
+            f0[a] -= v[a];
         }
+        slots[sid[c + 1]] = make_float4(v[0], v[1], v[2], 0.0f);
     }
-    float* out0 = d.slots + (size_t)sid[0] * 3;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) out0[a] = f0[a];
+    slots[sid[0]] = make_float4(f0[0], f0[1], f0[2], 0.0f);
 }
 
 // REF32: fem::stepCpu's node loop (fem.cpp:196-214).
-__global__ void __launch_bounds__(kBlock) ref32_nodes(TetDevice<float> d, float dt, float gravity,
+__global__ void __launch_bounds__(kTetNodeBlock) ref32_nodes(TetDevice<float> d, float dt, float gravity,
                                                       float damping) {
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= d.nodes) return;
@@ -260,14 +259,14 @@ __global__ void __launch_bounds__(kBlock) ref32_nodes(TetDevice<float> d, float 
     }
     const float m = d.mass[n];
     float force[3] = {0.0f, 0.0f, -gravity * m};
-    const uint32_t b = d.offset[n], e = d.offset[n + 1];
-    const float* sl = d.slots + (size_t)b * 3;
-#pragma unroll 4
-    for (uint32_t k = b; k < e; ++k, sl += 3) {
-        force[0] += sl[0];
-        force[1] += sl[1];
-        force[2] += sl[2];
-    }
+    const float4* slots = reinterpret_cast<const float4*>(d.slots);
+    for_run<8>(
+        slot_run(d.run[n]), [&](uint32_t k) { return slots[k]; },
+        [&](const float4& f) {
+            force[0] += f.x;
+            force[1] += f.y;
+            force[2] += f.z;
+        });
     const float inv_mass = 1.0f / m;
     float* pos = d.position + (size_t)n * 3;
 #pragma unroll
@@ -451,19 +450,21 @@ __global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d
         const uint4 sl = d.slot[t];
         const unsigned sid[4] = {sl.x, sl.y, sl.z, sl.w};
         double f0[3] = {0.0, 0.0, 0.0};
+        double2* xy = reinterpret_cast<double2*>(d.slots);
+        double* z = d.slots + 2 * d.slot_count;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            double* out = d.slots + (size_t)sid[c + 1] * 3;
+            double v[3];
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                const double v = scale * h(a, c);
-                out[a] = v;
-                f0[a] -= v;
+                v[a] = scale * h(a, c);
+                f0[a] -= v[a];
             }
+            xy[sid[c + 1]] = make_double2(v[0], v[1]);
+            z[sid[c + 1]] = v[2];
         }
-        double* out0 = d.slots + (size_t)sid[0] * 3;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) out0[a] = f0[a];
+        xy[sid[0]] = make_double2(f0[0], f0[1]);
+        z[sid[0]] = f0[2];
     }
     block_sum2(diss, energy, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
@@ -472,8 +473,8 @@ __global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d
     }
 }
 
-__global__ void __launch_bounds__(kBlock) f64_nodes(TetDevice<double> d, TetParams p) {
-    __shared__ double scratch[32];
+__global__ void __launch_bounds__(kTetNodeBlock) f64_nodes(TetDevice<double> d, TetParams p) {
+    __shared__ double scratch[64];
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double work = 0.0, kin = 0.0, gwork = 0.0;
     if (n < d.nodes) {
@@ -486,14 +487,19 @@ __global__ void __launch_bounds__(kBlock) f64_nodes(TetDevice<double> d, TetPara
             const double lf = ramp_factor(d.counter[1], p.ramp);
             const double m = d.mass[n];
             double force[3] = {0.0, 0.0, -p.gravity * m};
-            const uint32_t b = d.offset[n], e = d.offset[n + 1];
-            const double* sl = d.slots + (size_t)b * 3;
-#pragma unroll 4
-            for (uint32_t k = b; k < e; ++k, sl += 3) {
-                force[0] += sl[0];
-                force[1] += sl[1];
-                force[2] += sl[2];
-            }
+            const double2* xy = reinterpret_cast<const double2*>(d.slots);
+            const double* z = d.slots + 2 * d.slot_count;
+            for_run<8>(
+                slot_run(d.run[n]),
+                [&](uint32_t k) {
+                    const double2 f = xy[k];
+                    return make_double3(f.x, f.y, z[k]);
+                },
+                [&](const double3& f) {
+                    force[0] += f.x;
+                    force[1] += f.y;
+                    force[2] += f.z;
+                });
             double ext[3] = {0.0, 0.0, 0.0};
             if (d.ext) {
 #pragma unroll
@@ -515,13 +521,14 @@ __global__ void __launch_bounds__(kBlock) f64_nodes(TetDevice<double> d, TetPara
             gwork = -p.gravity * m * vel[2] * p.dt;
         }
     }
-    const double bw = block_sum(work, scratch);
-    const double bk = block_sum(kin, scratch);
-    const double bg = block_sum(gwork, scratch);
+    block_sum2(work, kin, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
-        d.n_work[blockIdx.x] += bw;
-        d.n_kin[blockIdx.x] = bk;
-        d.n_grav[blockIdx.x] += bg;
+        d.n_work[blockIdx.x] += work;
+        d.n_kin[blockIdx.x] = kin;
+    }
+    if (p.gravity != 0.0) {
+        gwork = block_sum(gwork, scratch);
+        if (threadIdx.x == 0) d.n_grav[blockIdx.x] += gwork;
     }
 }
 
@@ -673,13 +680,13 @@ void launch_ref32_step(const TetDevice<float>& d, const TetParams& p, cudaStream
     const float lambda = (float)p.lambda, mu = (float)p.mu;
     if (parts & kElementPart) ref32_forces<<<blocks_for(d.tets, kBlock), kBlock, 0, stream>>>(d, lambda, mu);
     if (parts & kNodePart)
-        ref32_nodes<<<blocks_for(d.nodes, kBlock), kBlock, 0, stream>>>(d, (float)p.dt, (float)p.gravity,
+        ref32_nodes<<<blocks_for(d.nodes, kTetNodeBlock), kTetNodeBlock, 0, stream>>>(d, (float)p.dt, (float)p.gravity,
                                                                          (float)p.damping);
 }
 
 void launch_f64_step(const TetDevice<double>& d, const TetParams& p, cudaStream_t stream, int parts) {
     if (parts & kElementPart) f64_forces<<<blocks_for(d.tets, kTet64Block), kTet64Block, 0, stream>>>(d, p);
-    if (parts & kNodePart) f64_nodes<<<blocks_for(d.nodes, kBlock), kBlock, 0, stream>>>(d, p);
+    if (parts & kNodePart) f64_nodes<<<blocks_for(d.nodes, kTetNodeBlock), kTetNodeBlock, 0, stream>>>(d, p);
 }
 
 void launch_tet_omega2(long long tets, const double* rest_inv, double E, double nu, double rho,

@@ -31,6 +31,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "tet.hpp"
 
 namespace fs {
 
@@ -384,7 +385,6 @@ __device__ __forceinline__ void tet_element_f32(const TetElementRefs& d, long lo
 }
 
 struct TetNodeRefs {
-    const uint32_t* offset;  // CSR offsets (absolute slot positions)
     const float4* slots;
     const uint8_t* fixed;
     const float* mass;
@@ -395,9 +395,11 @@ struct TetNodeRefs {
     float4* disp_c;          // compensated variant
 };
 
-// One node: CSR gather in order, external load, symplectic Euler on the displacement.
-template <bool KAHAN, bool CG = false>
-__device__ __forceinline__ void tet_node_f32(const TetNodeRefs& d, long long n, float lf, float dt, float gravity,
+// One node: its run of slots summed in order, external load, symplectic Euler on the
+// displacement.  BATCH slots' loads go out together; 0: a contiguous run, in the few
+// registers the pool's node pass has.
+template <bool KAHAN, bool CG = false, int BATCH = 8>
+__device__ __forceinline__ void tet_node_f32(const TetNodeRefs& d, const SlotRun& run, long long n, float lf, float dt, float gravity,
                                              float damping, double& work, double& kin, double& gwork) {
     work = kin = gwork = 0.0;
     float* vel = d.velocity + (size_t)n * 3;
@@ -409,13 +411,18 @@ __device__ __forceinline__ void tet_node_f32(const TetNodeRefs& d, long long n, 
     }
     const float m = d.mass[n];
     float force[3] = {0.0f, 0.0f, -gravity * m};
-    const uint32_t b = d.offset[n], e = d.offset[n + 1];
-#pragma unroll 4
-    for (uint32_t k = b; k < e; ++k) {
-        const float4 f = ldg_coherent4<CG>(d.slots + k);
+    const auto add = [&](const float4& f) {
         force[0] += f.x;
         force[1] += f.y;
         force[2] += f.z;
+    };
+    if constexpr (BATCH == 0) {
+        const uint32_t end = run.start + run.count;
+#pragma unroll 4
+        for (uint32_t k = run.start; k < end; ++k) add(ldg_coherent4<CG>(d.slots + k));
+    } else {
+        for_run<BATCH>(
+            run, [&](uint32_t k) { return ldg_coherent4<CG>(d.slots + k); }, add);
     }
     float ext[3] = {0.0f, 0.0f, 0.0f};
     if (d.ext) {

@@ -52,26 +52,27 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) f32_forces(TetDevice<fl
 }
 
 template <bool KAHAN>
-__global__ void __launch_bounds__(kBlock) f32_nodes(TetDevice<float> d, float dt, float gravity, float damping,
-                                                    int ramp) {
-    __shared__ double scratch[32];
+__global__ void __launch_bounds__(kTetNodeBlock) f32_nodes(TetDevice<float> d, float dt, float gravity, float damping,
+                                                           int ramp) {
+    __shared__ double scratch[64];
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double work = 0.0, kin = 0.0, gwork = 0.0;
     if (n < d.nodes) {
-        const TetNodeRefs r{d.offset,   reinterpret_cast<const float4*>(d.slots), d.fixed,
+        const TetNodeRefs r{reinterpret_cast<const float4*>(d.slots), d.fixed,
                             d.mass,     d.inv_mass,
                             d.ext,      d.velocity,
                             reinterpret_cast<float4*>(d.disp), reinterpret_cast<float4*>(d.disp_c)};
         const float lf = (float)ramp_factor(d.counter[1], ramp);
-        tet_node_f32<KAHAN>(r, n, lf, dt, gravity, damping, work, kin, gwork);
+        tet_node_f32<KAHAN>(r, slot_run(d.run[n]), n, lf, dt, gravity, damping, work, kin, gwork);
     }
-    const double bw = block_sum(work, scratch);
-    const double bk = block_sum(kin, scratch);
-    const double bg = block_sum(gwork, scratch);
+    block_sum2(work, kin, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
-        d.n_work[blockIdx.x] += bw;
-        d.n_kin[blockIdx.x] = bk;
-        d.n_grav[blockIdx.x] += bg;
+        d.n_work[blockIdx.x] += work;
+        d.n_kin[blockIdx.x] = kin;
+    }
+    if (gravity != 0.0f) {
+        gwork = block_sum(gwork, scratch);
+        if (threadIdx.x == 0) d.n_grav[blockIdx.x] += gwork;
     }
 }
 
@@ -79,17 +80,17 @@ __global__ void __launch_bounds__(kBlock) f32_nodes(TetDevice<float> d, float dt
 
 void launch_f32_step(const TetDevice<float>& d, const TetParams& p, bool compensated, cudaStream_t stream,
                      int parts) {
-    const int eb = blocks_for(d.tets, kBlock), nb = blocks_for(d.nodes, kBlock);
+    const int eb = blocks_for(d.tets, kBlock), nb = blocks_for(d.nodes, kTetNodeBlock);
     const J2f m = make_j2f(p.mu, p.bulk, p.yield, p.hardening);
     const int wave = sm_count() * (1024 / kBlock);
     if (compensated) {
         if (parts & kElementPart) f32_forces<true><<<eb, kBlock, 0, stream>>>(d, m, wave);
         if (parts & kNodePart)
-            f32_nodes<true><<<nb, kBlock, 0, stream>>>(d, (float)p.dt, (float)p.gravity, (float)p.damping, p.ramp);
+            f32_nodes<true><<<nb, kTetNodeBlock, 0, stream>>>(d, (float)p.dt, (float)p.gravity, (float)p.damping, p.ramp);
     } else {
         if (parts & kElementPart) f32_forces<false><<<eb, kBlock, 0, stream>>>(d, m, wave);
         if (parts & kNodePart)
-            f32_nodes<false><<<nb, kBlock, 0, stream>>>(d, (float)p.dt, (float)p.gravity, (float)p.damping, p.ramp);
+            f32_nodes<false><<<nb, kTetNodeBlock, 0, stream>>>(d, (float)p.dt, (float)p.gravity, (float)p.damping, p.ramp);
     }
 }
 

@@ -206,3 +206,34 @@ def test_f64_at_block_edges_and_large_rotations(fem, port, cells, pull):
     p, v = g.readback64()
     assert np.array_equal(p, ref.position) and np.array_equal(v, ref.velocity)
     assert np.array_equal(g.plastic().reshape(-1), ref.plastic)
+
+
+@pytest.mark.parametrize("spokes", [1, 7, 8, 9, 31, 300])
+def test_uneven_runs_of_slots(fem, port, spokes):
+    """A hub shared by every tet beside nodes of at most three: the node pass's runs are
+    strided where a group of 32 nodes is even and contiguous where it is not, and their
+    loads go in batches of eight.  FP64 and REF32 bit-identical to their oracles."""
+    k = np.arange(spokes + 2)
+    ring = np.stack([np.cos(2.1 * k), np.sin(2.1 * k), 0.3 * np.cos(0.7 * k)], 1)
+    pos = np.vstack([[[0.0, 0.0, 0.9]], ring]).astype(np.float32).reshape(-1)
+    idx = np.stack([0 * k[:-2], k[:-2] + 1, k[1:-1] + 1, k[2:] + 1], 1).astype(np.uint32).reshape(-1)
+    fixed = np.zeros(pos.size // 3, np.uint32)
+    fixed[-1] = 1
+    fext = np.zeros(pos.size)
+    fext[2] = 1e4
+    ref = O.TetMesh64(port, pos, idx, fixed, fext)
+    dt = port.tet64_critical_dt(C.byref(ref._s), 210e9, 0.3, 7850.0, 0.5)
+    ref.step(O.tet64_params(dt=dt, ramp_steps=10), 60)
+    g = fem.TetSolver(pos, idx, mode="f64", fixed=fixed, external_force=fext, density=7850.0)
+    g.run(60, dt=dt, ramp_steps=10)
+    p, v = g.readback64()
+    assert np.array_equal(p, ref.position) and np.array_equal(v, ref.velocity)
+    m = O.TetMesh32(port, pos, idx)
+    m.fixed[:] = fixed
+    m.rest_state(210e9, 0.3, 7850.0)
+    r = fem.TetSolver(pos, idx, mode="ref32", fixed=fixed, mass=m.mass, rest_inv=m.rest_inv,
+                      rest_volume=m.rest_volume, adjacency_offset=m.adj_offset, adjacency_entry=m.adj_entry)
+    m.step(210e9, 0.3, 7850.0, dt, 9.80665, 1.0, 60)
+    r.run(60, youngs=210e9, poisson=0.3, dt=dt, gravity=9.80665, damping=1.0)
+    pr, vr = r.readback()
+    assert np.array_equal(pr, m.position) and np.array_equal(vr, m.velocity)
