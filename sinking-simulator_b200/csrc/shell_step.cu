@@ -343,8 +343,6 @@ constexpr int kShellWarpsNarrow = kShellMinbNarrow * kShellBlock / 32;  // per S
 // double; 3 also alpha, its correction and its stored state (d.alpha64).
 template <bool KAHAN, bool GENERAL, int MINB, int EAS64 = 0>
 __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d, ShellParams p) {
-    // an inertial punch has stopped: the run is over (every thread reads the same flag)
-    if (d.halt && *d.halt) return;
     const int lane = threadIdx.x & 31;
     const int gp = lane & 7;
     const long long group_raw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -373,6 +371,13 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
             asm volatile("prefetch.global.L2 [%0];" ::"l"(d.elem + (at < last ? at : last)));
         }
     }
+    // what no step changes, while the pass before drains
+    const size_t og = (size_t)d.index[e * 8 + gp] * 3;
+    const double Xg = d.rest[og], Yg = d.rest[og + 1], Zg = d.rest[og + 2];
+    pdl_wait();
+    pdl_next();
+    // an inertial punch has stopped: the run is over (every thread reads the same flag)
+    if (d.halt && *d.halt) return;
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const long long s = d.counter[0];
         d.counter[1] = s;
@@ -391,8 +396,6 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     float dXg[3], ddg[3];
     {
         const int c0l = lane & 24;  // the lane of the element's corner 0
-        const size_t og = (size_t)d.index[e * 8 + gp] * 3;
-        const double Xg = d.rest[og], Yg = d.rest[og + 1], Zg = d.rest[og + 2];
         const float ug = d.disp[og], vg = d.disp[og + 1], wg = d.disp[og + 2];
         const double X0 = __shfl_sync(0xffffffffu, Xg, c0l), Y0 = __shfl_sync(0xffffffffu, Yg, c0l),
                      Z0 = __shfl_sync(0xffffffffu, Zg, c0l);
@@ -1076,14 +1079,19 @@ __device__ __forceinline__ void shell_move(float* u, float* uc, float v, float d
 template <bool KAHAN>
 __global__ void __launch_bounds__(kShellNodeBlock) shell_nodes(ShellDevice d, ShellParams p) {
     __shared__ double scratch[32];
-    if (d.halt && *d.halt) return;  // an inertial punch has stopped: the run is over
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long nr = n < d.nodes ? n : d.nodes - 1;
+    const uint32_t b = d.offset[nr], e = d.offset[nr + 1];
+    const uint8_t pin = d.pinned[nr];
+    const float im = d.inv_mass[nr], m = d.mass[nr];
+    pdl_wait();
+    pdl_next();
+    if (d.halt && *d.halt) return;  // an inertial punch has stopped: the run is over
     double work = 0.0, kin = 0.0, pwork = 0.0, damp = 0.0, bwork = 0.0;
     if (n < d.nodes) {
         const double t = (double)(d.counter[1] + 1) * p.dt64;  // the time at the step's end
         const float lf = p.rise_time > 0.0 ? (float)(t / p.rise_time < 1.0 ? t / p.rise_time : 1.0) : 1.0f;
         float force[3] = {0.0f, 0.0f, 0.0f};
-        const uint32_t b = d.offset[n], e = d.offset[n + 1];
         const float* sl = d.slots + (size_t)b * 3;
 #pragma unroll 4
         for (uint32_t k = b; k < e; ++k, sl += 3) {
@@ -1100,8 +1108,6 @@ __global__ void __launch_bounds__(kShellNodeBlock) shell_nodes(ShellDevice d, Sh
                 force[2] += fs[2];
             }
         }
-        const uint8_t pin = d.pinned[n];
-        const float im = d.inv_mass[n], m = d.mass[n];
         float* vel = d.velocity + (size_t)n * 3;
         float* u = d.disp + (size_t)n * 3;
         float* uc = d.disp_c + (size_t)n * 3;
@@ -1248,6 +1254,8 @@ __device__ __forceinline__ double fiber_return(const ShellParams::FiberLaw& m, d
 template <bool KAHAN>
 __global__ void __launch_bounds__(kShellFiberBlock) shell_fibers(ShellDevice d, ShellParams p) {
     __shared__ double scratch[64];
+    pdl_wait();
+    pdl_next();
     if (d.halt && *d.halt) return;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double diss = 0.0, energy = 0.0;
@@ -1325,6 +1333,8 @@ template <bool KAHAN>
 __global__ void __launch_bounds__(kShellPunchBlock) shell_punch(ShellDevice d, ShellParams p) {
     __shared__ double scratch[32];
     __shared__ double speed_s;
+    pdl_wait();
+    pdl_next();
     if (*d.halt) return;
     double momentum = 0.0, gripped_mass = 0.0;
     for (int i = threadIdx.x; i < d.n_driven; i += blockDim.x) {
@@ -1468,27 +1478,27 @@ static void launch_forces(const ShellDevice& d, const ShellParams& p, int blocks
     // the FP64 enhanced-block variants: compensated state and the general law only (the
     // host checks), at the narrow register budget
     if (p.eas64 == 1) {
-        shell_forces<true, true, kShellMinbNarrow, 1><<<blocks, kShellBlock, 0, stream>>>(d, p);
+        launch_pdl(shell_forces<true, true, kShellMinbNarrow, 1>, blocks, kShellBlock, 0, stream, d, p);
         return;
     }
     if (p.eas64 == 2) {
-        shell_forces<true, true, kShellMinbNarrow, 2><<<blocks, kShellBlock, 0, stream>>>(d, p);
+        launch_pdl(shell_forces<true, true, kShellMinbNarrow, 2>, blocks, kShellBlock, 0, stream, d, p);
         return;
     }
     if (p.eas64 == 3) {
-        shell_forces<true, true, kShellMinbNarrow, 3><<<blocks, kShellBlock, 0, stream>>>(d, p);
+        launch_pdl(shell_forces<true, true, kShellMinbNarrow, 3>, blocks, kShellBlock, 0, stream, d, p);
         return;
     }
     if (p.compensated) {
         if (p.general)
-            shell_forces<true, true, MINB><<<blocks, kShellBlock, 0, stream>>>(d, p);
+            launch_pdl(shell_forces<true, true, MINB>, blocks, kShellBlock, 0, stream, d, p);
         else
-            shell_forces<true, false, MINB><<<blocks, kShellBlock, 0, stream>>>(d, p);
+            launch_pdl(shell_forces<true, false, MINB>, blocks, kShellBlock, 0, stream, d, p);
     } else {
         if (p.general)
-            shell_forces<false, true, MINB><<<blocks, kShellBlock, 0, stream>>>(d, p);
+            launch_pdl(shell_forces<false, true, MINB>, blocks, kShellBlock, 0, stream, d, p);
         else
-            shell_forces<false, false, MINB><<<blocks, kShellBlock, 0, stream>>>(d, p);
+            launch_pdl(shell_forces<false, false, MINB>, blocks, kShellBlock, 0, stream, d, p);
     }
 }
 
@@ -1498,9 +1508,9 @@ void launch_shell_step(const ShellDevice& d, const ShellParams& p, cudaStream_t 
     const int fb = blocks_for(d.fibers, kShellFiberBlock);
     if ((parts & 1) && d.fibers) {
         if (p.compensated)
-            shell_fibers<true><<<fb, kShellFiberBlock, 0, stream>>>(d, p);
+            launch_pdl(shell_fibers<true>, fb, kShellFiberBlock, 0, stream, d, p);
         else
-            shell_fibers<false><<<fb, kShellFiberBlock, 0, stream>>>(d, p);
+            launch_pdl(shell_fibers<false>, fb, kShellFiberBlock, 0, stream, d, p);
     }
     // one wave at the narrow budget: the latency-bound form; else the wide one
     const bool narrow = d.groups <= (long long)d.sms * kShellWarpsNarrow;
@@ -1511,11 +1521,11 @@ void launch_shell_step(const ShellDevice& d, const ShellParams& p, cudaStream_t 
             launch_forces<kShellMinbWide>(d, p, eb, stream);
     }
     if (p.compensated) {
-        if (parts & 2) shell_nodes<true><<<nb, kShellNodeBlock, 0, stream>>>(d, p);
-        if ((parts & 2) && p.inertial) shell_punch<true><<<1, kShellPunchBlock, 0, stream>>>(d, p);
+        if (parts & 2) launch_pdl(shell_nodes<true>, nb, kShellNodeBlock, 0, stream, d, p);
+        if ((parts & 2) && p.inertial) launch_pdl(shell_punch<true>, 1, kShellPunchBlock, 0, stream, d, p);
     } else {
-        if (parts & 2) shell_nodes<false><<<nb, kShellNodeBlock, 0, stream>>>(d, p);
-        if ((parts & 2) && p.inertial) shell_punch<false><<<1, kShellPunchBlock, 0, stream>>>(d, p);
+        if (parts & 2) launch_pdl(shell_nodes<false>, nb, kShellNodeBlock, 0, stream, d, p);
+        if ((parts & 2) && p.inertial) launch_pdl(shell_punch<false>, 1, kShellPunchBlock, 0, stream, d, p);
     }
 }
 

@@ -194,22 +194,27 @@ __device__ __forceinline__ M3<double> polar_block(M3<double> r, bool live, Polar
 // REF32: fem::tetForces, written to the node-major slots.
 __global__ void __launch_bounds__(kBlock) ref32_forces(TetDevice<float> d, float lambda, float mu) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long tr = t < d.tets ? t : d.tets - 1;
+    const uint4 idx = d.index[tr], sl = d.slot[tr];
+    M3<float> dm_inv;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) dm_inv.m[k] = d.rest_inv[(size_t)k * d.tets + tr];
+    const float scale = -d.rest_vol[tr];
+    pdl_wait();
+    pdl_next();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const long long s = d.counter[0];
         d.counter[1] = s;
         d.counter[0] = s + 1;
     }
     if (t >= d.tets) return;
-    const uint4 idx = d.index[t];
     const unsigned nid[4] = {idx.x, idx.y, idx.z, idx.w};
     const float* p = d.position;
-    M3<float> ds, dm_inv;
+    M3<float> ds;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int a = 0; a < 3; ++a) ds(a, c) = p[(size_t)nid[c + 1] * 3 + a] - p[(size_t)nid[0] * 3 + a];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) dm_inv.m[k] = d.rest_inv[(size_t)k * d.tets + t];
     const M3<float> f = mul(ds, dm_inv);
     const M3<float> r = polar_fixed4(f);
     const M3<float> s = mul(transpose(r), f);
@@ -227,8 +232,6 @@ __global__ void __launch_bounds__(kBlock) ref32_forces(TetDevice<float> d, float
 #pragma unroll
     for (int i = 0; i < 3; ++i) stress(i, i) += lambda * trace;
     const M3<float> h = mul(mul(r, stress), transpose(dm_inv));
-    const float scale = -d.rest_vol[t];
-    const uint4 sl = d.slot[t];
     const unsigned sid[4] = {sl.x, sl.y, sl.z, sl.w};
     float f0[3] = {0.0f, 0.0f, 0.0f};
     float4* slots = reinterpret_cast<float4*>(d.slots);
@@ -249,19 +252,24 @@ __global__ void __launch_bounds__(kBlock) ref32_forces(TetDevice<float> d, float
 __global__ void __launch_bounds__(kTetNodeBlock) ref32_nodes(TetDevice<float> d, float dt, float gravity,
                                                       float damping) {
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long nr = n < d.nodes ? n : d.nodes - 1;
+    const SlotRun run = slot_run(d.run[nr]);
+    const float m = d.mass[nr];
+    const bool held = d.fixed[nr] != 0;
+    pdl_wait();
+    pdl_next();
     if (n >= d.nodes) return;
     float* vel = d.velocity + (size_t)n * 3;
-    if (d.fixed[n]) {
+    if (held) {
         vel[0] = 0.0f;
         vel[1] = 0.0f;
         vel[2] = 0.0f;
         return;
     }
-    const float m = d.mass[n];
     float force[3] = {0.0f, 0.0f, -gravity * m};
     const float4* slots = reinterpret_cast<const float4*>(d.slots);
     for_run<8>(
-        slot_run(d.run[n]), [&](uint32_t k) { return slots[k]; },
+        run, [&](uint32_t k) { return slots[k]; },
         [&](const float4& f) {
             force[0] += f.x;
             force[1] += f.y;
@@ -373,23 +381,28 @@ __global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d
     __shared__ double scratch[64];
     __shared__ PolarPark park;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = t < d.tets;
+    uint4 idx = make_uint4(0, 0, 0, 0);
+    if (live) {
+        idx = d.index[t];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) cp_async8(&park.rows[k][threadIdx.x], d.rest_inv + (size_t)k * d.tets + t);
+        cp_async_commit();
+        cp_async8(&park.rows[9][threadIdx.x], d.rest_vol + t);
+    }
+    pdl_wait();
+    pdl_next();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const long long s = d.counter[0];
         d.counter[1] = s;
         d.counter[0] = s + 1;
     }
     double diss = 0.0, energy = 0.0;
-    const bool live = t < d.tets;
     M3<double> f;
     if (live) {
-        const uint4 idx = d.index[t];
         const unsigned nid[4] = {idx.x, idx.y, idx.z, idx.w};
         const double* x = d.position;
         M3<double> ds, dm_inv;
-#pragma unroll
-        for (int k = 0; k < 9; ++k) cp_async8(&park.rows[k][threadIdx.x], d.rest_inv + (size_t)k * d.tets + t);
-        cp_async_commit();
-        cp_async8(&park.rows[9][threadIdx.x], d.rest_vol + t);
 #pragma unroll
         for (int i = 0; i < 7; ++i) cp_async8(&park.rows[10 + i][threadIdx.x], d.plastic + (size_t)i * d.tets + t);
         cp_async_commit();
@@ -477,6 +490,9 @@ __global__ void __launch_bounds__(kTetNodeBlock) f64_nodes(TetDevice<double> d, 
     __shared__ double scratch[64];
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double work = 0.0, kin = 0.0, gwork = 0.0;
+    const SlotRun run = slot_run(d.run[n < d.nodes ? n : d.nodes - 1]);
+    pdl_wait();
+    pdl_next();
     if (n < d.nodes) {
         double* vel = d.velocity + (size_t)n * 3;
         if (d.fixed[n]) {
@@ -490,7 +506,7 @@ __global__ void __launch_bounds__(kTetNodeBlock) f64_nodes(TetDevice<double> d, 
             const double2* xy = reinterpret_cast<const double2*>(d.slots);
             const double* z = d.slots + 2 * d.slot_count;
             for_run<8>(
-                slot_run(d.run[n]),
+                run,
                 [&](uint32_t k) {
                     const double2 f = xy[k];
                     return make_double3(f.x, f.y, z[k]);
@@ -678,15 +694,15 @@ void launch_widen(const float* in, long long n, double* out, cudaStream_t stream
 
 void launch_ref32_step(const TetDevice<float>& d, const TetParams& p, cudaStream_t stream, int parts) {
     const float lambda = (float)p.lambda, mu = (float)p.mu;
-    if (parts & kElementPart) ref32_forces<<<blocks_for(d.tets, kBlock), kBlock, 0, stream>>>(d, lambda, mu);
+    if (parts & kElementPart) launch_pdl(ref32_forces, blocks_for(d.tets, kBlock), kBlock, 0, stream, d, lambda, mu);
     if (parts & kNodePart)
-        ref32_nodes<<<blocks_for(d.nodes, kTetNodeBlock), kTetNodeBlock, 0, stream>>>(d, (float)p.dt, (float)p.gravity,
-                                                                         (float)p.damping);
+        launch_pdl(ref32_nodes, blocks_for(d.nodes, kTetNodeBlock), kTetNodeBlock, 0, stream, d, (float)p.dt,
+                   (float)p.gravity, (float)p.damping);
 }
 
 void launch_f64_step(const TetDevice<double>& d, const TetParams& p, cudaStream_t stream, int parts) {
-    if (parts & kElementPart) f64_forces<<<blocks_for(d.tets, kTet64Block), kTet64Block, 0, stream>>>(d, p);
-    if (parts & kNodePart) f64_nodes<<<blocks_for(d.nodes, kTetNodeBlock), kTetNodeBlock, 0, stream>>>(d, p);
+    if (parts & kElementPart) launch_pdl(f64_forces, blocks_for(d.tets, kTet64Block), kTet64Block, 0, stream, d, p);
+    if (parts & kNodePart) launch_pdl(f64_nodes, blocks_for(d.nodes, kTetNodeBlock), kTetNodeBlock, 0, stream, d, p);
 }
 
 void launch_tet_omega2(long long tets, const double* rest_inv, double E, double nu, double rho,

@@ -167,6 +167,26 @@ struct GlobalRows {
     __device__ __forceinline__ float plastic(int i, long long t) const { return d.plastic[(size_t)i * d.stride + t]; }
 };
 
+// The rows no step changes already in registers (loaded before the step's other data may
+// be touched), the plastic state from global memory.
+struct LoadedRows {
+    uint4 idx, slt;
+    float dm[9], v;
+    const TetElementRefs& d;
+    __device__ __forceinline__ LoadedRows(const TetElementRefs& refs, long long t) : d(refs) {
+        idx = refs.index[t];
+        slt = refs.slot[t];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) dm[k] = refs.rest_inv[(size_t)k * refs.stride + t];
+        v = refs.rest_vol[t];
+    }
+    __device__ __forceinline__ uint4 index(long long) const { return idx; }
+    __device__ __forceinline__ uint4 slot(long long) const { return slt; }
+    __device__ __forceinline__ float inv(int k, long long) const { return dm[k]; }
+    __device__ __forceinline__ float vol(long long) const { return v; }
+    __device__ __forceinline__ float plastic(int i, long long t) const { return d.plastic[(size_t)i * d.stride + t]; }
+};
+
 // A tile's rows in shared memory: index and slot map per tet from `first`, and 17
 // float rows (Dm^-1 0..8, volume 9, plastic state 10..16) of `pitch` floats each from
 // `base` (`first` rounded down to a multiple of 4, the 16-byte boundary of a row).

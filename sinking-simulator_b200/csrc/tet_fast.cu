@@ -35,15 +35,17 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) f32_forces(TetDevice<fl
         const long long ne = nb + blockDim.x < d.tets ? nb + blockDim.x : d.tets;
         prefetch_tet_rows(refs(d), nb, ne);
     }
+    const TetElementRefs r = refs(d);
+    const LoadedRows rows(r, t < d.tets ? t : d.tets - 1);
+    pdl_wait();
+    pdl_next();
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const long long s = d.counter[0];
         d.counter[1] = s;
         d.counter[0] = s + 1;
     }
     double diss = 0.0, energy = 0.0;
-    if (t < d.tets) {
-        tet_element_f32<KAHAN>(refs(d), t, m, diss, energy);
-    }
+    if (t < d.tets) tet_element_f32<KAHAN, false, LoadedRows>(r, rows, t, m, diss, energy);
     block_sum2(diss, energy, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
         d.e_diss[blockIdx.x] += diss;
@@ -57,13 +59,16 @@ __global__ void __launch_bounds__(kTetNodeBlock) f32_nodes(TetDevice<float> d, f
     __shared__ double scratch[64];
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double work = 0.0, kin = 0.0, gwork = 0.0;
+    const SlotRun run = slot_run(d.run[n < d.nodes ? n : d.nodes - 1]);
+    pdl_wait();
+    pdl_next();
     if (n < d.nodes) {
         const TetNodeRefs r{reinterpret_cast<const float4*>(d.slots), d.fixed,
                             d.mass,     d.inv_mass,
                             d.ext,      d.velocity,
                             reinterpret_cast<float4*>(d.disp), reinterpret_cast<float4*>(d.disp_c)};
         const float lf = (float)ramp_factor(d.counter[1], ramp);
-        tet_node_f32<KAHAN>(r, slot_run(d.run[n]), n, lf, dt, gravity, damping, work, kin, gwork);
+        tet_node_f32<KAHAN>(r, run, n, lf, dt, gravity, damping, work, kin, gwork);
     }
     block_sum2(work, kin, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
@@ -84,13 +89,15 @@ void launch_f32_step(const TetDevice<float>& d, const TetParams& p, bool compens
     const J2f m = make_j2f(p.mu, p.bulk, p.yield, p.hardening);
     const int wave = sm_count() * (1024 / kBlock);
     if (compensated) {
-        if (parts & kElementPart) f32_forces<true><<<eb, kBlock, 0, stream>>>(d, m, wave);
+        if (parts & kElementPart) launch_pdl(f32_forces<true>, eb, kBlock, 0, stream, d, m, wave);
         if (parts & kNodePart)
-            f32_nodes<true><<<nb, kTetNodeBlock, 0, stream>>>(d, (float)p.dt, (float)p.gravity, (float)p.damping, p.ramp);
+            launch_pdl(f32_nodes<true>, nb, kTetNodeBlock, 0, stream, d, (float)p.dt, (float)p.gravity, (float)p.damping,
+                       p.ramp);
     } else {
-        if (parts & kElementPart) f32_forces<false><<<eb, kBlock, 0, stream>>>(d, m, wave);
+        if (parts & kElementPart) launch_pdl(f32_forces<false>, eb, kBlock, 0, stream, d, m, wave);
         if (parts & kNodePart)
-            f32_nodes<false><<<nb, kTetNodeBlock, 0, stream>>>(d, (float)p.dt, (float)p.gravity, (float)p.damping, p.ramp);
+            launch_pdl(f32_nodes<false>, nb, kTetNodeBlock, 0, stream, d, (float)p.dt, (float)p.gravity,
+                       (float)p.damping, p.ramp);
     }
 }
 
