@@ -191,25 +191,25 @@ __global__ void __launch_bounds__(kTiledTile) pool_tile_fill(PoolDevice d, const
     }
 }
 
-// Dm^-1 (9 rows), the volume and the plastic state (7 rows)
-constexpr int kRowsPrefetched = 17;
-
-// L2 prefetch, by one warp (lane 0..31, a few lines each), of the rows the tiled pass
-// reads for tets [begin, end): the corner places (8 B per tet), Dm^-1 (9 rows of 4 B),
-// the volume and the plastic state (7 rows); every line starts inside its row's range.
-__device__ __forceinline__ void prefetch_tiled_rows_warp(const PoolDevice& d, long long begin, long long end,
-                                                         int lane) {
-    if (end <= begin) return;
-    const long long n = end - begin;
-    const int wide = (int)((n * 8 + 127) >> 7);
-    const int narrow = (int)((n * 4 + 127) >> 7);
-    for (int k = lane; k < wide; k += 32)
-        prefetch_l2(reinterpret_cast<const char*>(d.lidx + begin) + ((long long)k << 7));
-    for (int k = lane; k < kRowsPrefetched * narrow; k += 32) {
-        const int row = k / narrow, line = k - row * narrow;
+// L2 prefetch, one line a thread, of the rows the tiled pass reads for a tile's tets:
+// Dm^-1 (9 rows of 4 B a tet), the volume and the plastic state (7 rows) on threads 0-67,
+// the corner places and the sorted corners (8 B a tet each) on threads 68-83.  A line
+// starts inside its row's range.
+__device__ __forceinline__ void prefetch_tiled_rows(const PoolDevice& d, long long begin, long long end) {
+    const int n = (int)(end - begin);
+    int row = threadIdx.x >> 2, line = threadIdx.x & 3;
+    if (row < 17) {
+        if (line * 32 >= n) return;
         const float* rowp = row < 9 ? d.rest_inv + (size_t)row * d.tet_cap
                                     : (row == 9 ? d.rest_vol : d.plastic + (size_t)(row - 10) * d.tet_cap);
-        prefetch_l2(reinterpret_cast<const char*>(rowp + begin) + ((long long)line << 7));
+        prefetch_l2(rowp + begin + line * 32);
+    } else if (row < 21) {
+        line += 4 * ((row - 17) & 1);
+        if (line * 16 >= n) return;
+        if (row < 19)
+            prefetch_l2(d.lidx + begin + line * 16);
+        else
+            prefetch_l2(d.inv + 4 * (begin + line * 16));
     }
 }
 
@@ -247,77 +247,73 @@ struct TiledStage {
     }
 };
 
-// What a block needs of its tile, kept in shared memory by the fill that loaded it.
+// What a block needs of a tile: from the work list and the tables in one go, all loads
+// of it independent but the mesh's step.
 struct TiledInfo {
-    long long begin, end;
+    long long begin;
     uint32_t base;
-    int k, mesh, part, live;
+    int n, k, mesh, part;
+    __device__ __forceinline__ void load(const PoolDevice& d, int g) {
+        const PoolTile tl = d.etiles[g];
+        begin = tl.begin;
+        n = (int)(tl.end - tl.begin);
+        mesh = tl.mesh;
+        part = tl.part;
+        base = d.tab_off[g];
+        k = (int)d.tab_count[g];
+    }
+    __device__ __forceinline__ bool live(const PoolDevice& d, int sub) const {
+        const PoolMesh& m = d.meshes[mesh];
+        return m.step + sub < m.target;
+    }
 };
 
-// Queue the copies of tile g's gather and tables into `st` (every thread its share);
-// thread 0 records the tile in `info`.
-__device__ __forceinline__ void tiled_fill(const PoolDevice& d, int g, int sub, const TiledStage& st,
-                                           TiledInfo& info) {
-    const PoolTile tl = d.etiles[g];
-    const PoolMesh& m = d.meshes[tl.mesh];
-    const bool live = m.step + sub < m.target;
-    const uint32_t base = d.tab_off[g];
-    const int k = (int)d.tab_count[g];
-    if (threadIdx.x == 0) info = TiledInfo{tl.begin, tl.end, base, k, tl.mesh, tl.part, live ? 1 : 0};
-    if (!live) return;  // a frozen mesh's tile reads nothing
-    const int kp = (k + kTablePad - 1) / kTablePad * kTablePad;
-    for (int j = threadIdx.x; j < k; j += kTiledTile) {
-        const uint32_t n = d.node_tab[base + j];
+// Queue the copies of a tile's gather and tables into `st` (every thread its share);
+// `node` is this thread's entry of the tile's node list.
+__device__ __forceinline__ void tiled_fill(const PoolDevice& d, const TiledInfo& t, uint32_t node, const TiledStage& st) {
+    const int kp = (t.k + kTablePad - 1) / kTablePad * kTablePad;
+    for (int j = threadIdx.x; j < t.k; j += kTiledTile) {
+        const uint32_t n = j < kTiledTile ? node : d.node_tab[t.base + j];
         cp_async16(st.su + j, d.disp + n);
         cp_async16(st.sc + j, d.disp_c + n);
     }
     // the padded lists from their 16-byte aligned starts: 4 slots, or 8 starts, a copy
-    for (int q = threadIdx.x; q < kp / 4; q += kTiledTile) cp_async16(st.slot + 4 * q, d.part_slot + base + 4 * q);
+    for (int q = threadIdx.x; q < kp / 4; q += kTiledTile) cp_async16(st.slot + 4 * q, d.part_slot + t.base + 4 * q);
     for (int q = threadIdx.x; q < kp / 8; q += kTiledTile)
-        cp_async16(st.start + 8 * q, d.inv_start + base + 8 * q);
+        cp_async16(st.start + 8 * q, d.inv_start + t.base + 8 * q);
     // the sorted corners: four of them (8 bytes) per tet
-    const int n = (int)(tl.end - tl.begin);
-    if ((int)threadIdx.x < n) cp_async8(st.inv + 4 * threadIdx.x, d.inv + 4 * (tl.begin + threadIdx.x));
+    if ((int)threadIdx.x < t.n) cp_async8(st.inv + 4 * threadIdx.x, d.inv + 4 * (t.begin + threadIdx.x));
 }
 
+// The loop is ordered so that no load is waited for where it is issued: a tile's record
+// and its node ids are read two tiles ahead, during the node sums; its gather and tables
+// go out one tile ahead, before the evaluation; its tets' own rows are read into
+// registers during the node sums of the tile before, where few others are needed.  Two
+// barriers a tile: one that ends the wait for the gather (and the last tile's node sums,
+// whose stage is then refilled), one between the corner forces and the node sums.  The
+// tile's energy sums are left per warp and added up after the next barrier.  The pass is
+// bound by latency and the L1 pipe together (issue 62 %, L1 72 % busy, 8 blocks of 64
+// registers an SM; 6, 7 and 9 blocks: 516, 494 and 500 us for 458).  256 meshes, 10.99 M
+// tets: 491 us with the record, ids and rows read where they were used and four barriers,
+// 458 us so; 128 threads, each with its tet's 18 values, are more warps than two tets a
+// thread would leave.
 __global__ void __launch_bounds__(kTiledTile, 1024 / kTiledTile) pool_elements_tiled_ring(PoolDevice d, int sub,
                                                                                           int kcap) {
     extern __shared__ __align__(16) unsigned char tiled_smem[];
     __shared__ float4 sf[kTiledCorners];  // corner c of tet i at c x 128 + i
-    __shared__ double scratch[64];
+    __shared__ double warp_sums[2][2][kTiledTile / 32];
     __shared__ TiledInfo info[2];
+    __shared__ int is_live[2];
     const int G = (int)gridDim.x;
     int g = blockIdx.x;
     if (g >= d.n_etiles) return;
     const TiledStage st0(tiled_smem, kcap), st1(tiled_smem + TiledStage::bytes(kcap), kcap);
-    tiled_fill(d, g, sub, st0, info[0]);
-    cp_async_commit();
-    for (int it = 0;; ++it) {
-        const TiledStage& cur = (it & 1) ? st1 : st0;
-        const TiledStage& oth = (it & 1) ? st0 : st1;
-        const int nxt = g + G;
-        // the tile after next into L2, its rows and tables, by the last warp alone
-        if (threadIdx.x >= kTiledTile - 32 && nxt + G < d.n_etiles) {
-            const PoolTile nx = d.etiles[nxt + G];
-            const int lane = threadIdx.x - (kTiledTile - 32);
-            prefetch_tiled_rows_warp(d, nx.begin, nx.end, lane);
-            const uint32_t ob = d.tab_off[nxt + G];
-            if (lane == 0) prefetch_l2(d.node_tab + ob);
-            if (lane == 1) prefetch_l2(d.part_slot + ob);
-            if (lane == 2) prefetch_l2(d.inv_start + ob);
-        }
-        // this tile, as its fill recorded it: visible after the barriers of the tile before
-        // (its wait), or, for the first tile, after this one
-        if (it == 0) __syncthreads();
-        const TiledInfo& ti = info[it & 1];
-        const PoolMesh& m = d.meshes[ti.mesh];
-        const bool live = ti.live != 0;
-        const long long t = ti.begin + threadIdx.x;
-        const bool mine = live && t < ti.end;
-        // this tet's rows and corner places into registers (their latency overlaps the wait)
-        RegRows rr;
-        ushort4 l = make_ushort4(0, 0, 0, 0);
-        if (mine) {
+    // this tet's rows and corner places in its tile
+    RegRows rr;
+    ushort4 l = make_ushort4(0, 0, 0, 0);
+    const auto load_rows = [&](long long begin, int n, bool live) {
+        if (live && (int)threadIdx.x < n) {
+            const long long t = begin + threadIdx.x;
             l = d.lidx[t];
 #pragma unroll
             for (int q = 0; q < 9; ++q) rr.dm[q] = d.rest_inv[(size_t)q * d.tet_cap + t];
@@ -325,33 +321,85 @@ __global__ void __launch_bounds__(kTiledTile, 1024 / kTiledTile) pool_elements_t
 #pragma unroll
             for (int i = 0; i < 7; ++i) rr.pl[i] = d.plastic[(size_t)i * d.tet_cap + t];
         }
-        // the next tile's copies go out now; this tile's have landed once all but the
-        // newest group are done, in every thread
-        if (nxt < d.n_etiles) tiled_fill(d, nxt, sub, oth, info[(it & 1) ^ 1]);
+    };
+    // a finished tile's account: its warps' sums in warp order
+    const auto close_tile = [&](int which) {
+        if (threadIdx.x == 0 && is_live[which]) {
+            double diss = 0.0, energy = 0.0;
+#pragma unroll
+            for (int w = 0; w < kTiledTile / 32; ++w) {
+                diss += warp_sums[which][0][w];
+                energy += warp_sums[which][1][w];
+            }
+            d.e_diss[info[which].part] += diss;
+            d.e_strain[info[which].part] = energy;
+        }
+    };
+    TiledInfo next;  // the tile after the one in hand: its record, this thread's node of it, its mesh live
+    uint32_t node = 0;
+    bool next_live;
+    {
+        TiledInfo first;
+        first.load(d, g);
+        const bool live = first.live(d, sub);
+        if ((int)threadIdx.x < first.k) node = d.node_tab[first.base + threadIdx.x];
+        if (threadIdx.x == 0) {
+            info[0] = first;
+            is_live[0] = live ? 1 : 0;
+        }
+        if (live) tiled_fill(d, first, node, st0);  // a frozen mesh's tile reads nothing
         cp_async_commit();
-        cp_async_wait_one();
+        load_rows(first.begin, first.n, live);
+        next.load(d, g + G < d.n_etiles ? g + G : g);
+        next_live = next.live(d, sub);
+        if ((int)threadIdx.x < next.k) node = d.node_tab[next.base + threadIdx.x];
+    }
+    for (int it = 0;; ++it) {
+        const int b = it & 1;
+        const TiledStage& cur = b ? st1 : st0;
+        cp_async_wait_all();
         __syncthreads();
+        if (it > 0) close_tile(b ^ 1);
+        const bool more = g + G < d.n_etiles;
+        if (more) {
+            if (next_live) tiled_fill(d, next, node, b ? st0 : st1);
+            cp_async_commit();
+            if (threadIdx.x == 0) {
+                info[b ^ 1] = next;
+                is_live[b ^ 1] = next_live ? 1 : 0;
+            }
+        }
+        const int after = g + 2 * G;
+        if (after < d.n_etiles) {
+            const PoolTile nx = d.etiles[after];
+            prefetch_tiled_rows(d, nx.begin, nx.end);
+        }
+        const bool live = is_live[b] != 0;
         double diss = 0.0, energy = 0.0;
-        if (mine) {
+        if (live && (int)threadIdx.x < info[b].n) {
             const float4 un[4] = {cur.su[l.x], cur.su[l.y], cur.su[l.z], cur.su[l.w]};
             const float4 cn[4] = {cur.sc[l.x], cur.sc[l.y], cur.sc[l.z], cur.sc[l.w]};
             const TetElementRefs r{d.index,     d.slot, d.rest_inv, d.rest_vol, d.plastic,
                                    d.plastic_c, d.disp, d.disp_c,   d.slots,    d.tet_cap};
             float4 fc[4];
-            tet_element_f32_eval<true, RegRows>(r, rr, t, m.mat, un, cn, diss, energy, fc);
+            tet_element_f32_eval<true, RegRows>(r, rr, info[b].begin + threadIdx.x, d.meshes[info[b].mesh].mat, un, cn,
+                                                diss, energy, fc);
             sf[threadIdx.x] = fc[0];
             sf[kTiledTile + threadIdx.x] = fc[1];
             sf[2 * kTiledTile + threadIdx.x] = fc[2];
             sf[3 * kTiledTile + threadIdx.x] = fc[3];
         }
         __syncthreads();
+        if (more) {
+            load_rows(info[b ^ 1].begin, info[b ^ 1].n, is_live[b ^ 1] != 0);
+            next.load(d, after < d.n_etiles ? after : g);
+        }
         if (live) {
-            const int k = ti.k;
-            const int corners = 4 * (int)(ti.end - ti.begin);
+            const int k = info[b].k, corners = 4 * info[b].n;
             for (int j = threadIdx.x; j < k; j += kTiledTile) {
-                const int b = cur.start[j], e = j + 1 < k ? cur.start[j + 1] : corners;
-                float4 f = sf[cur.inv[b]];
-                for (int q = b + 1; q < e; ++q) {
+                const int s = cur.start[j], e = j + 1 < k ? cur.start[j + 1] : corners;
+                float4 f = sf[cur.inv[s]];
+                for (int q = s + 1; q < e; ++q) {
                     const float4 h = sf[cur.inv[q]];
                     f.x += h.x;
                     f.y += h.y;
@@ -360,15 +408,20 @@ __global__ void __launch_bounds__(kTiledTile, 1024 / kTiledTile) pool_elements_t
                 d.slots[cur.slot[j]] = make_float4(f.x, f.y, f.z, 0.0f);
             }
         }
-        block_sum2(diss, energy, scratch);  // valid in thread 0; also ends the stage's reads
-        if (live && threadIdx.x == 0) {
-            d.e_diss[ti.part] += diss;
-            d.e_strain[ti.part] = energy;
+        warp_sum2(diss, energy);
+        if ((threadIdx.x & 31) == 0) {
+            warp_sums[b][0][threadIdx.x >> 5] = diss;
+            warp_sums[b][1][threadIdx.x >> 5] = energy;
         }
-        if (nxt >= d.n_etiles) break;
-        g = nxt;
+        if (!more) {
+            __syncthreads();
+            close_tile(b);
+            break;
+        }
+        next_live = next.live(d, sub);
+        if ((int)threadIdx.x < next.k) node = d.node_tab[next.base + threadIdx.x];
+        g += G;
     }
-    cp_async_wait_all();
 }
 
 }  // namespace

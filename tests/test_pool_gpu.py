@@ -467,3 +467,35 @@ def test_tiled_schedule_refuses_other_tile_sizes(fem):
     pool.run(15)
     assert pool.status(0) == (20, 20)
     pool.close()
+
+
+@pytest.mark.parametrize("cells", [(22, 1, 1), (11, 5, 4)])
+def test_tiled_schedule_on_shuffled_tets(fem, cells):
+    """Tets in random order: a tile's corners then name up to 512 distinct nodes (a box
+    mesh's about 90), so the gather and the node sums take several rounds.  132 tets (a
+    second tile of four) and 1,320; beside a mesh that finishes early and freezes.
+    Within 1e-6 of the graph schedule."""
+    rng = np.random.default_rng(5)
+    nx, ny, nz = cells
+    pos, idx = fem.box_tet_mesh(0.05 * nx, 0.05 * ny, 0.05 * nz, nx, ny, nz)
+    idx = idx.reshape(-1, 4)[rng.permutation(idx.size // 4)].reshape(-1)
+    fixed = (pos[0::3] < 1e-6).astype(np.uint32)
+    tip = pos[0::3] > 0.05 * nx - 1e-6
+    fext = np.zeros(pos.size)
+    fext[2::3][tip] = -3e4 / tip.sum()
+    mesh = dict(position=pos, index=idx, fixed=fixed, external_force=fext, density=7850.0, youngs=210e9, poisson=0.3,
+                yield_strength=235e6, hardening=1e9, ramp_steps=100)
+    out = {}
+    for mode in (fem.POOL_GRAPH, fem.POOL_GRAPH_TILED):
+        pool = fem.TetPool(20000, 8000, max_meshes=4, tile=128)
+        pool.set_schedule(128, mode)
+        short, i = pool.admit_many([mesh, mesh], [50, 300])
+        pool.run(300)
+        out[mode] = [pool.readback(short)[0], pool.readback(i)[0], pool.energy(i)]
+        pool.close()
+    for k in (0, 1):
+        a, b = out[fem.POOL_GRAPH][k], out[fem.POOL_GRAPH_TILED][k]
+        assert np.abs(a - pos).max() > 1e-7
+        assert np.abs(a - b).max() <= 1e-6 * np.abs(a - pos).max()
+    e, f = out[fem.POOL_GRAPH][2], out[fem.POOL_GRAPH_TILED][2]
+    assert np.abs(e - f).max() <= 1e-6 * abs(e[0])
