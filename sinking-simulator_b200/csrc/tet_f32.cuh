@@ -205,114 +205,6 @@ struct SharedRows {
     }
 };
 
-// The rotation's deviation Q = R - I and the co-rotated strain U - I (engineering shears)
-// of F = I + H = R U, from the displacement gradient H.
-//
-// At a small stretch, by series: with B = (H + H^T + H^T H) / 2 = (U^2 - I) / 2 exactly, its
-// square root E = U - I by the fixed point E <- B - E^2 / 2 from E = B, and Q by
-// Q <- X - Q E from Q = X = H - E (from R U = F).  Each round gains a factor |E|: after
-// n rounds E is off by |E|^(n+2) / 2 and Q by |X| |E|^(n+1), so two rounds reach FP32's
-// precision at elastic strains and three up to |E| of about 1e-2.  Beyond, by the Higham
-// iteration Q <- (Q - (M Q)^T) / 2, M = (I + Q)^-1 (fem.cpp:62-69), which squares the
-// stretch error and halves it: three steps up to 0.1, the reference's four beyond.
-// The series has no divide and, in two rounds, 160 operations against 300 for two Higham
-// steps and R^T F (a tiled element pass of 3.9 M tets: 127 M -> 109 M warp instructions).
-// The squares are summed apart, so an entry of E takes one rounding at its own size:
-// at rotations of 1e-3 to 0.5 rad the strain's relative error is 0.1 to 1 of what it was
-// as R^T F - I (5.6e-7 for 4.8e-6 at 0.1 rad and a strain of 1e-3), and where nothing
-// rotates 4.5e-8 for 3.7e-8; the solvers' errors against 64 bits are unchanged or smaller.
-constexpr float kSeriesTwo = 1.25e-3f, kSeriesThree = 6e-3f;  // on the largest entry of B
-
-// One round: E <- B - E^2 / 2.
-__device__ __forceinline__ void series_round(const float (&b)[6], float (&e)[6]) {
-    // entries xx yy zz xy yz zx
-    const float xx = e[0], yy = e[1], zz = e[2], xy = e[3], yz = e[4], zx = e[5];
-    e[0] = __fmaf_rn(-0.5f, __fmaf_rn(zx, zx, __fmaf_rn(xy, xy, xx * xx)), b[0]);
-    e[1] = __fmaf_rn(-0.5f, __fmaf_rn(yz, yz, __fmaf_rn(xy, xy, yy * yy)), b[1]);
-    e[2] = __fmaf_rn(-0.5f, __fmaf_rn(zx, zx, __fmaf_rn(yz, yz, zz * zz)), b[2]);
-    e[3] = __fmaf_rn(-0.5f, __fmaf_rn(zx, yz, __fmaf_rn(xy, yy, xx * xy)), b[3]);
-    e[4] = __fmaf_rn(-0.5f, __fmaf_rn(yz, zz, __fmaf_rn(yy, yz, xy * zx)), b[4]);
-    e[5] = __fmaf_rn(-0.5f, __fmaf_rn(zz, zx, __fmaf_rn(yz, xy, zx * xx)), b[5]);
-}
-
-// Q <- X - Q E.
-__device__ __forceinline__ void series_rotate(const M3<float>& x, const float (&e)[6], M3<float>& q) {
-    const int at[3][3] = {{0, 3, 5}, {3, 1, 4}, {5, 4, 2}};
-    M3<float> r;
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-            r(i, j) = __fmaf_rn(-q(i, 2), e[at[2][j]], __fmaf_rn(-q(i, 1), e[at[1][j]], __fmaf_rn(-q(i, 0), e[at[0][j]], x(i, j))));
-    q = r;
-}
-
-__device__ __forceinline__ void tet_polar_f32(const M3<float>& h, M3<float>& q, float (&strain)[6]) {
-    float b[6];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const int j = (i + 1) % 3;
-        b[i] = __fmaf_rn(0.5f, __fmaf_rn(h(2, i), h(2, i), __fmaf_rn(h(1, i), h(1, i), h(0, i) * h(0, i))), h(i, i));
-        b[3 + i] = 0.5f * ((h(i, j) + h(j, i)) +
-                           __fmaf_rn(h(2, i), h(2, j), __fmaf_rn(h(1, i), h(1, j), h(0, i) * h(0, j))));
-    }
-    const float big = fmaxf(fmaxf(fmaxf(fabsf(b[0]), fabsf(b[1])), fmaxf(fabsf(b[2]), fabsf(b[3]))),
-                            fmaxf(fabsf(b[4]), fabsf(b[5])));
-    if (big <= kSeriesThree) {
-        float e[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) e[i] = b[i];
-        series_round(b, e);
-        series_round(b, e);
-        const bool third = big > kSeriesTwo;
-        if (third) series_round(b, e);
-        const M3<float> x = [&] {
-            M3<float> d = h;
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const int j = (i + 1) % 3;
-                d(i, i) -= e[i];
-                d(i, j) -= e[3 + i];
-                d(j, i) -= e[3 + i];
-            }
-            return d;
-        }();
-        q = x;
-        series_rotate(x, e, q);
-        series_rotate(x, e, q);
-        if (third) series_rotate(x, e, q);
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            strain[i] = e[i];
-            strain[3 + i] = 2.0f * e[3 + i];
-        }
-        return;
-    }
-    const int higham_steps = big <= 0.1f ? 3 : 4;
-    q = h;
-#pragma unroll 1
-    for (int it = 0; it < higham_steps; ++it) {
-        M3<float> ipq = q;
-        ipq(0, 0) += 1.0f;
-        ipq(1, 1) += 1.0f;
-        ipq(2, 2) += 1.0f;
-        const M3<float> mq = mul_fma(inverse_fma(ipq, 1e-30f), q);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) ipq(i, j) = 0.5f * (q(i, j) - mq(j, i));
-        q = ipq;
-    }
-    const M3<float> qt = transpose(q);
-    const M3<float> qth = mul_fma(qt, h);
-    strain[0] = h(0, 0) + qt(0, 0) + qth(0, 0);
-    strain[1] = h(1, 1) + qt(1, 1) + qth(1, 1);
-    strain[2] = h(2, 2) + qt(2, 2) + qth(2, 2);
-    strain[3] = (h(0, 1) + qt(0, 1) + qth(0, 1)) + (h(1, 0) + qt(1, 0) + qth(1, 0));
-    strain[4] = (h(1, 2) + qt(1, 2) + qth(1, 2)) + (h(2, 1) + qt(2, 1) + qth(2, 1));
-    strain[5] = (h(2, 0) + qt(2, 0) + qth(2, 0)) + (h(0, 2) + qt(0, 2) + qth(0, 2));
-}
-
 // One tet from its four corners' displacements un (and compensations cn), however
 // they were fetched: its four corner forces into fc (x, y, z, 0), its plastic state
 // advanced; the dissipation and strain energy of the element in diss / energy (FP64,
@@ -337,9 +229,37 @@ __device__ __forceinline__ void tet_element_f32_eval(const TetElementRefs& d, co
 #pragma unroll
     for (int k = 0; k < 9; ++k) dm_inv.m[k] = rows.inv(k, t);
     const M3<float> h = mul_fma(du, dm_inv);  // displacement gradient
-    M3<float> q;
+    // rotation deviation Q = R - I by the Higham iteration on F = I + H.  Each step
+    // squares the stretch error and halves it (F = R (I + E) goes to R (I + E^2 / 2)),
+    // starting from about |sym H|, so the steps to reach FP32's relative precision of
+    // the strain itself are known before the first: two up to |sym H| = 8e-3, three up
+    // to 0.1, the reference's four beyond (fem.cpp:62-69 always takes four).
+    const float e0 = fmaxf(fmaxf(fmaxf(fabsf(h(0, 0)), fabsf(h(1, 1))), fmaxf(fabsf(h(2, 2)), fabsf(h(0, 1) + h(1, 0)))),
+                           fmaxf(fabsf(h(1, 2) + h(2, 1)), fabsf(h(2, 0) + h(0, 2))));
+    const int higham_steps = e0 <= 8e-3f ? 2 : (e0 <= 0.1f ? 3 : 4);
+    M3<float> q = h;
+#pragma unroll 1
+    for (int it = 0; it < higham_steps; ++it) {
+        M3<float> ipq = q;
+        ipq(0, 0) += 1.0f;
+        ipq(1, 1) += 1.0f;
+        ipq(2, 2) += 1.0f;
+        const M3<float> mq = mul_fma(inverse_fma(ipq, 1e-30f), q);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) ipq(i, j) = 0.5f * (q(i, j) - mq(j, i));
+        q = ipq;
+    }
+    const M3<float> qt = transpose(q);
+    const M3<float> qth = mul_fma(qt, h);
     float strain[6];
-    tet_polar_f32(h, q, strain);
+    strain[0] = h(0, 0) + qt(0, 0) + qth(0, 0);
+    strain[1] = h(1, 1) + qt(1, 1) + qth(1, 1);
+    strain[2] = h(2, 2) + qt(2, 2) + qth(2, 2);
+    strain[3] = (h(0, 1) + qt(0, 1) + qth(0, 1)) + (h(1, 0) + qt(1, 0) + qth(1, 0));
+    strain[4] = (h(1, 2) + qt(1, 2) + qth(1, 2)) + (h(2, 1) + qt(2, 1) + qth(2, 1));
+    strain[5] = (h(2, 0) + qt(2, 0) + qth(2, 0)) + (h(0, 2) + qt(0, 2) + qth(0, 2));
 
     // radial return, linear isotropic hardening (plasticity.cpp:333-456); for a linear
     // curve the consistency condition is affine in dgamma and its root is the closed
@@ -352,33 +272,23 @@ __device__ __forceinline__ void tet_element_f32_eval(const TetElementRefs& d, co
     for (int i = 0; i < 6; ++i) el[i] = strain[i] - ps[i];
     const float vol_strain = el[0] + el[1] + el[2];
     const float pressure = m.kappa * vol_strain;
-    const float two_mu = 2.0f * m.mu, third = vol_strain * (1.0f / 3.0f);
     float trial[6];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        trial[i] = two_mu * (el[i] - third);
+        trial[i] = 2.0f * m.mu * (el[i] - vol_strain * (1.0f / 3.0f));
         trial[3 + i] = m.mu * el[3 + i];
     }
-    const float shear2 = __fmaf_rn(trial[5], trial[5], __fmaf_rn(trial[4], trial[4], trial[3] * trial[3]));
-    const float norm2 = __fmaf_rn(
-        2.0f, shear2, __fmaf_rn(trial[2], trial[2], __fmaf_rn(trial[1], trial[1], trial[0] * trial[0])));
+    const float norm = sqrtf(trial[0] * trial[0] + trial[1] * trial[1] + trial[2] * trial[2] +
+                             2.0f * (trial[3] * trial[3] + trial[4] * trial[4] + trial[5] * trial[5]));
     const float root23 = 0.81649658092772603f;
-    const float radius = root23 * __fmaf_rn(m.hardening, fmaxf(ps[6], 0.0f), m.yield);
-    // an elastic tet needs no square root: norm > radius is decided on the squares
-    float norm = 0.0f, excess = 0.0f;
-    if (norm2 > radius * fabsf(radius)) {
-        norm = sqrtf(norm2);
-        excess = norm - radius;
-    }
-    float dev = norm2;  // s : s of the final stress, for the energy
+    const float radius = root23 * (m.yield + m.hardening * fmaxf(ps[6], 0.0f));
+    const float excess = norm - radius;
     float sv[6];
     diss = 0.0;
     if (excess > 0.0f) {
-        const float gamma = excess / __fmaf_rn(2.0f / 3.0f, m.hardening, two_mu);
+        const float gamma = excess / (2.0f * m.mu + (2.0f / 3.0f) * m.hardening);
         const float inv_norm = 1.0f / norm;
-        const float k = two_mu * gamma * inv_norm;
-        const float left = __fmaf_rn(-two_mu, gamma, norm);
-        dev = left * left;
+        const float k = 2.0f * m.mu * gamma * inv_norm;
         float dp[6];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
@@ -421,30 +331,41 @@ __device__ __forceinline__ void tet_element_f32_eval(const TetElementRefs& d, co
     }
     const float volf = rows.vol(t);
     diss *= (double)volf;
-    // 1/2 sigma : C^-1 : sigma = 1/2 [s : s / (2 mu) + p tr(sigma) / (3 kappa)], tr(sigma) =
-    // 3 p, the engineering shears counted twice in s : s; the density in FP32 (a relative
-    // error of a few ulps per tet), the account summed in FP64
-    energy = (double)(volf * 0.5f * __fmaf_rn(dev, m.inv_2mu_f, 3.0f * pressure * pressure * m.inv_3kappa_f));
-    // P = R sigma = sigma + Q sigma; nodal forces f_c = -V (P Dm^-T) column c, with -V
-    // taken into sigma
+    {
+        // 1/2 sigma : C^-1 : sigma = 1/2 [s_dev : s_dev / (2 mu) + p tr(sigma) / (3 kappa)]
+        // with p = tr(sigma) / 3, the engineering shears counted twice; the density in
+        // FP32 (a relative error of a few ulps per tet), the account summed in FP64
+        const float tr = sv[0] + sv[1] + sv[2];
+        const float pr = tr * (1.0f / 3.0f);
+        const float d0 = sv[0] - pr, d1 = sv[1] - pr, d2 = sv[2] - pr;
+        const float dev = d0 * d0 + d1 * d1 + d2 * d2 + 2.0f * (sv[3] * sv[3] + sv[4] * sv[4] + sv[5] * sv[5]);
+        energy = (double)(volf * 0.5f * (dev * m.inv_2mu_f + pr * tr * m.inv_3kappa_f));
+    }
+    // P = R sigma = sigma + Q sigma; nodal forces f_c = -V (P Dm^-T) column c
+    M3<float> sig;
+    sig(0, 0) = sv[0];
+    sig(1, 1) = sv[1];
+    sig(2, 2) = sv[2];
+    sig(0, 1) = sig(1, 0) = sv[3];
+    sig(1, 2) = sig(2, 1) = sv[4];
+    sig(2, 0) = sig(0, 2) = sv[5];
+    const M3<float> qs = mul_fma(q, sig);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) sig.m[k] += qs.m[k];
+    const M3<float> hf = mul_fma(sig, transpose(dm_inv));
     const float scale = -volf;
-    M3<float> sig, pk;
-    sig(0, 0) = scale * sv[0];
-    sig(1, 1) = scale * sv[1];
-    sig(2, 2) = scale * sv[2];
-    sig(0, 1) = sig(1, 0) = scale * sv[3];
-    sig(1, 2) = sig(2, 1) = scale * sv[4];
-    sig(2, 0) = sig(0, 2) = scale * sv[5];
+    float f0[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
+    for (int c = 0; c < 3; ++c) {
+        float v[3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
-            pk(i, c) = __fmaf_rn(q(i, 2), sig(2, c), __fmaf_rn(q(i, 1), sig(1, c), __fmaf_rn(q(i, 0), sig(0, c), sig(i, c))));
-    const M3<float> hf = mul_fma(pk, transpose(dm_inv));
-#pragma unroll
-    for (int c = 0; c < 3; ++c) fc[c + 1] = make_float4(hf(0, c), hf(1, c), hf(2, c), 0.0f);
-    fc[0] = make_float4(-hf(0, 0) - hf(0, 1) - hf(0, 2), -hf(1, 0) - hf(1, 1) - hf(1, 2),
-                        -hf(2, 0) - hf(2, 1) - hf(2, 2), 0.0f);
+        for (int a = 0; a < 3; ++a) {
+            v[a] = scale * hf(a, c);
+            f0[a] -= v[a];
+        }
+        fc[c + 1] = make_float4(v[0], v[1], v[2], 0.0f);
+    }
+    fc[0] = make_float4(f0[0], f0[1], f0[2], 0.0f);
 }
 
 // The same with the corner forces written to the node-major slots (one 16-byte store
