@@ -1470,7 +1470,7 @@ int femstep_pool_profile(femstep_pool* p, int steps, double out[2]) {
         else
             fs::launch_pool_element_pass(p->d, p->tile, s, p->stream, p->mode == FEMSTEP_POOL_GRAPH_STAGED);
         cudaEventRecord(ev[1], p->stream);
-        fs::launch_pool_node_pass(dn, p->tile, s, p->stream);
+        fs::launch_pool_node_pass(dn, p->tile, s, p->stream, tiled);
         cudaEventRecord(ev[2], p->stream);
         rc = check(p, cudaEventSynchronize(ev[2]), "profile");
         float a = 0.0f, b = 0.0f;

@@ -51,7 +51,8 @@ struct PoolDevice {
     float* rest_vol = nullptr;
     float* plastic = nullptr;
     float* plastic_c = nullptr;
-    float4* slots = nullptr;       // 4 per tet capacity: (fx, fy, fz, 0) per corner
+    float4* slots = nullptr;       // 4 per tet capacity: (fx, fy, fz, 0) per corner; the corners of a
+                                   // mesh's 32 consecutive nodes share one stretch, in jagged order
     // nodes
     uint32_t* offset = nullptr;    // [node_cap]: CSR begin of each node; every mesh holds
                                    // one spare node slot after its last node for the end
@@ -105,9 +106,10 @@ enum class PoolPasses { kDirect, kStaged, kTiled };
 // Two launches per step (element, node), `steps` times, then the advance, on `stream`.
 void launch_pool_steps(const PoolDevice& d, int tile, int steps, cudaStream_t stream, PoolPasses passes);
 // The passes one at a time (per-kernel timing): element or node pass of sub-step
-// `sub`, and the advance by `steps`.
+// `sub`, and the advance by `steps`.  `tiled`: the node pass reads the tiled schedule's
+// partials (d.offset set to part_off) instead of the corners' slots.
 void launch_pool_element_pass(const PoolDevice& d, int tile, int sub, cudaStream_t stream, bool staged);
-void launch_pool_node_pass(const PoolDevice& d, int tile, int sub, cudaStream_t stream);
+void launch_pool_node_pass(const PoolDevice& d, int tile, int sub, cudaStream_t stream, bool tiled);
 void launch_pool_advance(const PoolDevice& d, int steps, cudaStream_t stream);
 // One persistent cooperative launch for `steps` steps on `blocks` co-resident blocks,
 // then the advance.

@@ -415,12 +415,11 @@ struct TetNodeRefs {
     float4* disp_c;          // compensated variant
 };
 
-// One node: its run of slots summed in order, external load, symplectic Euler on the
-// displacement.  BATCH slots' loads go out together; 0: a contiguous run, in the few
-// registers the pool's node pass has.
-template <bool KAHAN, bool CG = false, int BATCH = 8>
-__device__ __forceinline__ void tet_node_f32(const TetNodeRefs& d, const SlotRun& run, long long n, float lf, float dt, float gravity,
-                                             float damping, double& work, double& kin, double& gwork) {
+// One node: `gather` adds the forces of its slots in order to its weight (it is not called
+// for a fixed node); external load, symplectic Euler on the displacement.
+template <bool KAHAN, class Gather>
+__device__ __forceinline__ void tet_node_f32(const TetNodeRefs& d, Gather gather, long long n, float lf, float dt,
+                                             float gravity, float damping, double& work, double& kin, double& gwork) {
     work = kin = gwork = 0.0;
     float* vel = d.velocity + (size_t)n * 3;
     if (d.fixed[n]) {
@@ -431,19 +430,7 @@ __device__ __forceinline__ void tet_node_f32(const TetNodeRefs& d, const SlotRun
     }
     const float m = d.mass[n];
     float force[3] = {0.0f, 0.0f, -gravity * m};
-    const auto add = [&](const float4& f) {
-        force[0] += f.x;
-        force[1] += f.y;
-        force[2] += f.z;
-    };
-    if constexpr (BATCH == 0) {
-        const uint32_t end = run.start + run.count;
-#pragma unroll 4
-        for (uint32_t k = run.start; k < end; ++k) add(ldg_coherent4<CG>(d.slots + k));
-    } else {
-        for_run<BATCH>(
-            run, [&](uint32_t k) { return ldg_coherent4<CG>(d.slots + k); }, add);
-    }
+    gather(force);
     float ext[3] = {0.0f, 0.0f, 0.0f};
     if (d.ext) {
 #pragma unroll

@@ -68,7 +68,16 @@ __global__ void __launch_bounds__(kTetNodeBlock) f32_nodes(TetDevice<float> d, f
                             d.ext,      d.velocity,
                             reinterpret_cast<float4*>(d.disp), reinterpret_cast<float4*>(d.disp_c)};
         const float lf = (float)ramp_factor(d.counter[1], ramp);
-        tet_node_f32<KAHAN>(r, run, n, lf, dt, gravity, damping, work, kin, gwork);
+        const auto gather = [&](float(&force)[3]) {
+            for_run<8>(
+                run, [&](uint32_t k) { return r.slots[k]; },
+                [&](const float4& f) {
+                    force[0] += f.x;
+                    force[1] += f.y;
+                    force[2] += f.z;
+                });
+        };
+        tet_node_f32<KAHAN>(r, gather, n, lf, dt, gravity, damping, work, kin, gwork);
     }
     block_sum2(work, kin, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {

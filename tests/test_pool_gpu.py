@@ -499,3 +499,32 @@ def test_tiled_schedule_on_shuffled_tets(fem, cells):
         assert np.abs(a - b).max() <= 1e-6 * np.abs(a - pos).max()
     e, f = out[fem.POOL_GRAPH][2], out[fem.POOL_GRAPH_TILED][2]
     assert np.abs(e - f).max() <= 1e-6 * abs(e[0])
+
+
+@pytest.mark.parametrize("spokes", [1, 7, 30, 31, 300])
+@pytest.mark.parametrize("mode", [1, 2, 3])
+def test_uneven_nodes_bit_identical_to_single_mesh_step(fem, spokes, mode):
+    """A hub shared by every tet beside nodes of one to three, 4 to 303 nodes: the jagged
+    slots of a warp's nodes, with a ragged last warp, in the graph, persistent and staged
+    schedules, beside another mesh; bit-identical to the single-mesh step."""
+    k = np.arange(spokes + 2)
+    ring = np.stack([np.cos(2.1 * k), np.sin(2.1 * k), 0.3 * np.cos(0.7 * k)], 1)
+    pos = np.vstack([[[0.0, 0.0, 0.9]], ring]).astype(np.float32).reshape(-1)
+    idx = np.stack([0 * k[:-2], k[:-2] + 1, k[1:-1] + 1, k[2:] + 1], 1).astype(np.uint32).reshape(-1)
+    fixed = np.zeros(pos.size // 3, np.uint32)
+    fixed[-1] = 1
+    fext = np.zeros(pos.size)
+    fext[2] = 1e5
+    s = fem.TetSolver(pos, idx, mode="f32k", fixed=fixed, external_force=fext, density=7850.0)
+    dt = s.critical_dt(safety=0.5)
+    s.run(60, dt=dt, ramp_steps=10, gravity=9.80665)
+    p, v = s.readback64()
+    pool = fem.TetPool(4000, 2000, max_meshes=4, tile=128)
+    pool.set_schedule(128, mode)
+    hub = dict(position=pos, index=idx, fixed=fixed, external_force=fext, dt=dt, ramp_steps=10, gravity=9.80665)
+    ids = pool.admit_many([hub, dict(hub, fixed=None), hub], [60, 60, 60])
+    pool.run(60)
+    for i in (ids[0], ids[2]):
+        q, w = pool.readback(i)
+        assert np.array_equal(p, q) and np.array_equal(v, w)
+    pool.close()
