@@ -308,7 +308,7 @@ __device__ __forceinline__ void point_law_general(const float eps[6], const floa
 
 // C g for the algorithmic tangent C = kappa 1(x)1 + 2 mu theta I_dev - 2 mu thetaBar n(x)n
 // in the reference's Voigt convention (engineering strain in, tensor stress out).
-__device__ __forceinline__ void tangent_apply(const PointOut& o, const ShellParams& p, const float g[6], float out[6]) {
+__device__ __forceinline__ void tangent_apply(const PointOut& o, float kappa, float mu, const float g[6], float out[6]) {
     if (o.failed) {  // a failed point carries nothing
 #pragma unroll
         for (int i = 0; i < 6; ++i) out[i] = 0.0f;
@@ -316,11 +316,85 @@ __device__ __forceinline__ void tangent_apply(const PointOut& o, const ShellPara
     }
     const float tr = g[0] + g[1] + g[2];
     const float ng = o.n[0] * g[0] + o.n[1] * g[1] + o.n[2] * g[2] + o.n[3] * g[3] + o.n[4] * g[4] + o.n[5] * g[5];
-    const float a = 2.0f * p.mu * o.theta, b = 2.0f * p.mu * o.theta_bar * ng;
+    const float a = 2.0f * mu * o.theta, b = 2.0f * mu * o.theta_bar * ng;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) out[i] = p.kappa * tr + a * (g[i] - tr * (1.0f / 3.0f)) - b * o.n[i];
+    for (int i = 0; i < 3; ++i) out[i] = kappa * tr + a * (g[i] - tr * (1.0f / 3.0f)) - b * o.n[i];
 #pragma unroll
     for (int i = 3; i < 6; ++i) out[i] = 0.5f * a * g[i] - b * o.n[i];
+}
+
+// K_aa = sum_g w_g G^T C G of the lane's element (the whole warp calls it) from the lane's
+// tangent (flow direction, theta, theta-bar), and its Cholesky factor, lower triangle
+// with the diagonal as its reciprocal, into `factor` (the element's, in shared memory);
+// whether it is positive definite.  Not inlined: only warps with a yielded point come
+// here, and inlined its hundred registers spilled values of every step.
+__device__ __noinline__ bool shell_tangent_factor(float n0, float n1, float n2, float n3, float n4, float n5, float theta,
+                                                  float theta_bar, bool failed, float gc0, float gc1, float gc2, float gc3,
+                                                  float gc4, float gc5, float gc6, float w, float kappa, float mu,
+                                                  const float* T, float* factor) {
+    PointOut o;
+    o.n[0] = n0;
+    o.n[1] = n1;
+    o.n[2] = n2;
+    o.n[3] = n3;
+    o.n[4] = n4;
+    o.n[5] = n5;
+    o.theta = theta;
+    o.theta_bar = theta_bar;
+    o.failed = failed;
+    const float gc[7] = {gc0, gc1, gc2, gc3, gc4, gc5, gc6};
+    float l[28];
+    bool spd = true;
+    // K_aa = sum_g w_g G^T C G, lower triangle: with G factored, the point's part is
+    // gc_a gc_b H[k_a][k_b], H = T0c^T C T0c over T0's four columns (four tangent
+    // applications rather than seven)
+    float kaa[28];
+    {
+        float H[10];
+#pragma unroll
+        for (int kb = 0; kb < 4; ++kb) {
+            float cg[6];
+            tangent_apply(o, kappa, mu, &T[kb * 6], cg);
+#pragma unroll
+            for (int ka = kb; ka < 4; ++ka) {
+                float s = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 6; ++i) s += T[ka * 6 + i] * cg[i];
+                H[ka * (ka + 1) / 2 + kb] = w * s;
+            }
+        }
+        const int kj[7] = {0, 1, 2, 2, 2, 3, 3};
+#pragma unroll
+        for (int b = 0; b < 7; ++b)
+#pragma unroll
+            for (int a = b; a < 7; ++a)
+                kaa[a * (a + 1) / 2 + b] = sum8(gc[a] * gc[b] * H[kj[a] * (kj[a] + 1) / 2 + kj[b]]);
+    }
+    // Cholesky (solid_shell.cpp:432-457), identical in every lane
+    {
+        int t = 0;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) {
+#pragma unroll
+            for (int j = 0; j <= i; ++j) {
+                float s = kaa[t];
+#pragma unroll
+                for (int k = 0; k < j; ++k) s -= l[i * (i + 1) / 2 + k] * l[j * (j + 1) / 2 + k];
+                if (i == j) {  // the diagonal is kept as its reciprocal
+                    spd = spd && (s > 0.0f);
+                    l[t] = 1.0f / sqrtf(fmaxf(s, 1e-30f));
+                } else {
+                    l[t] = s * l[j * (j + 1) / 2 + j];
+                }
+                ++t;
+            }
+        }
+    }
+    if ((threadIdx.x & 7) == 0) {
+#pragma unroll
+        for (int k = 0; k < 28; ++k) factor[k] = l[k];
+    }
+    return spd;
 }
 
 // Blocks per SM the register budget is sized for, chosen per launch.  With the
@@ -695,82 +769,35 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
             }
             if (__all_sync(0xffffffffu, done)) break;
         }
-        float l[28];
+        // The factor of each element goes to its record in shared memory, from where the
+        // substitutions read it row by row: 28 registers fewer in every lane.
         bool spd = true;
+        float* factor = geo + kGeoL;
+        __syncwarp();
         if (__any_sync(0xffffffffu, !elastic_element)) {
-        // K_aa = sum_g w_g G^T C G, lower triangle: with G factored, the point's part is
-        // gc_a gc_b H[k_a][k_b], H = T0c^T C T0c over T0's four columns (four tangent
-        // applications rather than seven)
-        float kaa[28];
-        {
-            float H[10];
-#pragma unroll
-            for (int kb = 0; kb < 4; ++kb) {
-                float cg[6];
-                tangent_apply(o, p, &T[kb * 6], cg);
-#pragma unroll
-                for (int ka = kb; ka < 4; ++ka) {
-                    float s = 0.0f;
-#pragma unroll
-                    for (int i = 0; i < 6; ++i) s += T[ka * 6 + i] * cg[i];
-                    H[ka * (ka + 1) / 2 + kb] = w * s;
-                }
-            }
-            const int kj[7] = {0, 1, 2, 2, 2, 3, 3};
-#pragma unroll
-            for (int b = 0; b < 7; ++b)
-#pragma unroll
-                for (int a = b; a < 7; ++a)
-                    kaa[a * (a + 1) / 2 + b] = sum8(gc[a] * gc[b] * H[kj[a] * (kj[a] + 1) / 2 + kj[b]]);
+            const bool ok = shell_tangent_factor(o.n[0], o.n[1], o.n[2], o.n[3], o.n[4], o.n[5], o.theta, o.theta_bar, o.failed,
+                                                 gc[0], gc[1], gc[2], gc[3], gc[4], gc[5], gc[6], w, p.kappa, p.mu, T, factor);
+            spd = elastic_element || ok;
+            __syncwarp();
         }
-        // Cholesky (solid_shell.cpp:432-457), identical in every lane
-        {
-            int t = 0;
-#pragma unroll
-            for (int i = 0; i < 7; ++i) {
-#pragma unroll
-                for (int j = 0; j <= i; ++j) {
-                    float s = kaa[t];
-#pragma unroll
-                    for (int k = 0; k < j; ++k) s -= l[i * (i + 1) / 2 + k] * l[j * (j + 1) / 2 + k];
-                    if (i == j) {  // the diagonal is kept as its reciprocal
-                        spd = spd && (s > 0.0f);
-                        l[t] = 1.0f / sqrtf(fmaxf(s, 1e-30f));
-                    } else {
-                        l[t] = s * l[j * (j + 1) / 2 + j];
-                    }
-                    ++t;
-                }
-            }
-        }
-        }
-        if (elastic_element && !done) {
-            const float4* lf = reinterpret_cast<const float4*>(d.kaa_factor + e * 32);
-#pragma unroll
-            for (int k = 0; k < 7; ++k) {
-                const float4 v = __ldg(lf + k);
-                l[4 * k] = v.x;
-                l[4 * k + 1] = v.y;
-                l[4 * k + 2] = v.z;
-                l[4 * k + 3] = v.w;
-            }
-            spd = true;
-        }
+        if (elastic_element && !done && gp < 7)
+            reinterpret_cast<float4*>(factor)[gp] = __ldg(reinterpret_cast<const float4*>(d.kaa_factor + e * 32) + gp);
+        __syncwarp();
         // L L^T delta = -r; the factor's diagonal holds 1 / l_ii
         float delta[7];
 #pragma unroll
         for (int i = 0; i < 7; ++i) {
             float s = -r[i];
 #pragma unroll
-            for (int k = 0; k < i; ++k) s -= l[i * (i + 1) / 2 + k] * delta[k];
-            delta[i] = s * l[i * (i + 1) / 2 + i];
+            for (int k = 0; k < i; ++k) s -= factor[i * (i + 1) / 2 + k] * delta[k];
+            delta[i] = s * factor[i * (i + 1) / 2 + i];
         }
 #pragma unroll
         for (int i = 6; i >= 0; --i) {
             float s = delta[i];
 #pragma unroll
-            for (int k = i + 1; k < 7; ++k) s -= l[k * (k + 1) / 2 + i] * delta[k];
-            delta[i] = s * l[i * (i + 1) / 2 + i];
+            for (int k = i + 1; k < 7; ++k) s -= factor[k * (k + 1) / 2 + i] * delta[k];
+            delta[i] = s * factor[i * (i + 1) / 2 + i];
         }
         float work = 0.0f;
 #pragma unroll
@@ -832,7 +859,7 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
 #pragma unroll
                     for (int kb = 0; kb < 4; ++kb) {
                         float cg[6];
-                        tangent_apply(o, p, &T[kb * 6], cg);
+                        tangent_apply(o, p.kappa, p.mu, &T[kb * 6], cg);
 #pragma unroll
                         for (int ka = kb; ka < 4; ++ka) {
                             double s = 0.0;
@@ -852,7 +879,7 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
 #pragma unroll
                     for (int kb = 0; kb < 4; ++kb) {
                         float cg[6];
-                        tangent_apply(o, p, &T[kb * 6], cg);
+                        tangent_apply(o, p.kappa, p.mu, &T[kb * 6], cg);
 #pragma unroll
                         for (int ka = kb; ka < 4; ++ka) {
                             float s = 0.0f;
