@@ -70,6 +70,19 @@ __device__ __forceinline__ void kahan_add(float& sum, float& comp, float x) {
     sum = t;
 }
 
+// N floats (a multiple of four) of an element's record in shared memory, 16 bytes a load.
+template <int N>
+__device__ __forceinline__ void load_record(const float* from, float* to) {
+#pragma unroll
+    for (int k = 0; k < N / 4; ++k) {
+        const float4 v = reinterpret_cast<const float4*>(from)[k];
+        to[4 * k] = v.x;
+        to[4 * k + 1] = v.y;
+        to[4 * k + 2] = v.z;
+        to[4 * k + 3] = v.w;
+    }
+}
+
 // Element e's rest corners for the element operators: the bottom corners relative to
 // corner 0 and the directors D_c = X_{c+4} - X_c, each difference taken in double and
 // rounded once (the same values the step forms from its own node loads).
@@ -448,10 +461,38 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     // what no step changes, while the pass before drains
     const size_t og = (size_t)d.index[e * 8 + gp] * 3;
     const double Xg = d.rest[og], Yg = d.rest[og + 1], Zg = d.rest[og + 2];
+    // The element row (J0^-1 and the enhanced-mode scales) and the points' start-of-step
+    // state are wanted only after the corners' chain of loads and the rotation.  The wide
+    // form, short of registers, has them copied into shared memory meanwhile, the state
+    // staying there through the Newton iterations; so do its frames, between the strain
+    // and the forces.  The narrow form has registers for all of it, and forms the frame again.
+    constexpr bool PARK = MINB >= kShellMinbWide;
+    constexpr int kParkLanes = PARK ? kShellBlock : 1;
+    const int park = PARK ? threadIdx.x : 0;
+    __shared__ __align__(16) float4 row_park[PARK ? kShellBlock / 8 : 1][kShellElemQ];
+    __shared__ float ps_park[7][kParkLanes], frame_park[15][kParkLanes];
+    const size_t sbase = (size_t)group * kShellStateQ * 32 + lane;
+    float ps_reg[7];
+    if constexpr (PARK) {
+        if (gp < kShellElemQ) cp_async16(&row_park[threadIdx.x >> 3][gp], d.elem + e * kShellElemQ + gp);
+        cp_async_commit();
+    }
     pdl_wait();
     pdl_next();
     // an inertial punch has stopped: the run is over (every thread reads the same flag)
-    if (d.halt && *d.halt) return;
+    if (d.halt && *d.halt) {
+        if (PARK) cp_async_wait_all();
+        return;
+    }
+    if constexpr (PARK) {
+#pragma unroll
+        for (int k = 0; k < 7; ++k) cp_async4(&ps_park[k][park], d.state + sbase + (size_t)k * 32);
+        cp_async_commit();
+    }
+    const auto start_state = [&](float (&ps)[7]) {
+#pragma unroll
+        for (int k = 0; k < 7; ++k) ps[k] = PARK ? ps_park[k][park] : ps_reg[k];
+    };
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const long long s = d.counter[0];
         d.counter[1] = s;
@@ -510,11 +551,15 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
         }
         __syncwarp();
     }
-    // ---- the element row: J0^-1 and the enhanced-mode scales (all zero: no valid forms) ----
     float j0[9], cm[7];
     {
         const float4* row = d.elem + e * kShellElemQ;
-        const float4 r0 = __ldg(row), r1 = __ldg(row + 1), r2 = __ldg(row + 2), r3 = __ldg(row + 3);
+        if constexpr (PARK) {
+            cp_async_wait_one();  // the row's copies, by four of the element's lanes
+            __syncwarp();
+            row = row_park[threadIdx.x >> 3];
+        }
+        const float4 r0 = row[0], r1 = row[1], r2 = row[2], r3 = row[3];
         const float v[16] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
 #pragma unroll
         for (int k = 0; k < 9; ++k) j0[k] = v[k];
@@ -527,6 +572,8 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     // ---- rotation: H = (sum_a dN_a(0) (x) dd_a) J0^-1, R = I + Q ----
     float q[9];
     {
+        float dd[24];
+        load_record<24>(geo + kGeoDd, dd);
         const float sx[8] = {-1, 1, 1, -1, -1, 1, 1, -1}, sy[8] = {-1, -1, 1, 1, -1, -1, 1, 1},
                     sz[8] = {-1, -1, -1, -1, 1, 1, 1, 1};
         float jd[9];
@@ -535,7 +582,7 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
             float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
 #pragma unroll
             for (int a = 0; a < 8; ++a) {
-                const float v = geo[kGeoDd + a * 3 + i];
+                const float v = dd[a * 3 + i];
                 a0 += sx[a] * v;
                 a1 += sy[a] * v;
                 a2 += sz[a] * v;
@@ -593,9 +640,6 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
             geo[kGeoU + gp * 3 + i] = ddg[i] + (q[0 * 3 + i] * sx + q[1 * 3 + i] * ty + q[2 * 3 + i] * wz);
         __syncwarp();
     }
-    const float(*dX)[3] = reinterpret_cast<const float(*)[3]>(geo + kGeoX);
-    const float(*D)[3] = reinterpret_cast<const float(*)[3]>(geo + kGeoD);
-    const float* u = geo + kGeoU;
 
     // the rotation waits in shared memory through the Newton iterations (each lane its
     // own copy: no synchronisation), freeing nine registers there
@@ -604,10 +648,24 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     for (int k = 0; k < 9; ++k) q_park[k][threadIdx.x] = q[k];
     // ---- the point's operators, formed from the rest geometry ----
     const ShellLanePoint P = shell_lane_point(gp);
-    float gx[3], gy[3], Ainv[9], w;
-    shell_frame(dX, D, P, formed, gx, gy, Ainv, w);
-    float eps_u[6];
-    shell_strain(dX, D, u, P, gx, gy, Ainv, eps_u);
+    float w, eps_u[6];
+    {
+        float dX[4][3], D[4][3], u[24], gx[3], gy[3], Ainv[9];
+        load_record<12>(geo + kGeoX, &dX[0][0]);
+        load_record<12>(geo + kGeoD, &D[0][0]);
+        shell_frame(dX, D, P, formed, gx, gy, Ainv, w);
+        if constexpr (PARK) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                frame_park[k][park] = gx[k];
+                frame_park[3 + k][park] = gy[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 9; ++k) frame_park[6 + k][park] = Ainv[k];
+        }
+        load_record<24>(geo + kGeoU, u);
+        shell_strain(dX, D, u, P, gx, gy, Ainv, eps_u);
+    }
     // G factored: column j = gc_j T0[:, k_j], k = (0, 1, 2, 2, 2, 3, 3)
     // T0 is the element's, the same in its eight lanes: one copy in the element's record
     // in shared memory rather than 24 registers in every lane through the Newton loop
@@ -632,10 +690,12 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     gnorm = sqrtf(gnorm);
 
     // ---- start-of-step state ----
-    const size_t sbase = (size_t)group * kShellStateQ * 32 + lane;
-    float ps[7];
+    if constexpr (PARK) {
+        cp_async_wait_all();  // each lane its own
+    } else {
 #pragma unroll
-    for (int k = 0; k < 7; ++k) ps[k] = d.state[sbase + (size_t)k * 32];
+        for (int k = 0; k < 7; ++k) ps_reg[k] = d.state[sbase + (size_t)k * 32];
+    }
     float back0[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, damage0 = 0.0f, fstrain = INFINITY;
     bool failed0 = false;
     const size_t sbase2 = (size_t)group * kShellState2Q * 32 + lane;
@@ -650,8 +710,13 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     bool eas_on = true;
     if (GENERAL) eas_on = ((__ballot_sync(0xffffffffu, failed0) >> (lane & 24)) & 0xffu) == 0u;
     float alpha[7];
+    {
+        const float4* row = reinterpret_cast<const float4*>(d.alpha + e * 8);
+        const float4 a = row[0], b = row[1];
+        const float v[7] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z};
 #pragma unroll
-    for (int k = 0; k < 7; ++k) alpha[k] = eas_on ? d.alpha[e * 8 + k] : 0.0f;
+        for (int k = 0; k < 7; ++k) alpha[k] = eas_on ? v[k] : 0.0f;
+    }
     double alpha64[7];
     if constexpr (EAS64 >= 3) {
 #pragma unroll
@@ -676,6 +741,8 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
                 shell_enhanced_apply64(T, gc, alpha64, eps_u, eps);
             else
                 shell_enhanced_apply(T, gc, alpha, eps_u, eps);
+            float ps[7];
+            start_state(ps);
             if (GENERAL)
                 point_law_general(eps, ps, back0, damage0, failed0, fstrain, p, o);
             else
@@ -832,7 +899,7 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
                     const float s0 = sn[0] - pr, s1 = sn[1] - pr, s2 = sn[2] - pr;
                     const float norm =
                         sqrtf(s0 * s0 + s1 * s1 + s2 * s2 + 2.0f * (sn[3] * sn[3] + sn[4] * sn[4] + sn[5] * sn[5]));
-                    const float radius = 0.81649658092772603f * (p.yield + p.hardening * fmaxf(ps[6], 0.0f));
+                    const float radius = 0.81649658092772603f * (p.yield + p.hardening * fmaxf(PARK ? ps_park[6][park] : ps_reg[6], 0.0f));
                     linear_try = true;
                     linear_elastic = norm <= radius;
                 }
@@ -978,6 +1045,8 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
                 shell_enhanced_apply64(T, gc, alpha64, eps_u, eps);
             else
                 shell_enhanced_apply(T, gc, alpha, eps_u, eps);
+            float ps[7];
+            start_state(ps);
             point_law_general(eps, ps, back0, damage0, failed0, fstrain, p, o);
         }
     }
@@ -990,6 +1059,8 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     if (valid) {
         if (o.yielded) {
             diss = (double)w * (double)o.diss;
+            float ps[7];
+            start_state(ps);
             if (KAHAN) {
                 // the compensations are read only here, where a yielded point needs them
                 float pc[7];
@@ -1033,14 +1104,25 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     }
 
     // ---- f = -R sum_g w_g B_g^T sigma_g, reduce-scattered so lane a holds node a ----
-    // (the rest corners back from shared memory and the point's frame formed again:
-    // cheaper than holding them in registers through the Newton iterations)
+    const uint32_t slot = d.slot[e * 8 + gp];
     float f[24];
 #pragma unroll
     for (int j = 0; j < 24; ++j) f[j] = 0.0f;
     {
-        float fx[3], fy[3], Af[9], wf;
-        shell_frame(dX, D, P, formed, fx, fy, Af, wf);
+        float dX[4][3], D[4][3], fx[3], fy[3], Af[9], wf = w;
+        load_record<12>(geo + kGeoX, &dX[0][0]);
+        load_record<12>(geo + kGeoD, &D[0][0]);
+        if constexpr (PARK) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                fx[k] = frame_park[k][park];
+                fy[k] = frame_park[3 + k][park];
+            }
+#pragma unroll
+            for (int k = 0; k < 9; ++k) Af[k] = frame_park[6 + k][park];
+        } else {
+            shell_frame(dX, D, P, formed, fx, fy, Af, wf);
+        }
         shell_force(dX, D, P, fx, fy, Af, wf, o.sigma, f);
     }
     // round 1 (xor 4): keep nodes 0-3 (bit 2 clear) or 4-7
@@ -1065,7 +1147,7 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     }
     if (valid) {
         // lane gp now holds sum over points of node gp's internal force; apply -R
-        float* out = d.slots + (size_t)d.slot[e * 8 + gp] * 3;
+        float* out = d.slots + (size_t)slot * 3;
         float qr[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) qr[k] = q_park[k][threadIdx.x];
@@ -1076,15 +1158,17 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     // elements converge early does not wait for the slowest warp of its block
     const unsigned nonconv = __ballot_sync(0xffffffffu, valid && gp == 0 && !converged);
     const unsigned ypts = __ballot_sync(0xffffffffu, valid && o.yielded);
+    if (ypts) {  // else the dissipation is zero in every lane
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        diss += __shfl_xor_sync(0xffffffffu, diss, off);
-        energy += __shfl_xor_sync(0xffffffffu, energy, off);
+        for (int off = 16; off > 0; off >>= 1) diss += __shfl_xor_sync(0xffffffffu, diss, off);
     }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) energy += __shfl_xor_sync(0xffffffffu, energy, off);
     if (lane == 0) {
-        d.e_diss[group_raw] += diss;
+        // sums that gain nothing stand as they are, unread
+        if (diss != 0.0) d.e_diss[group_raw] += diss;
         d.e_strain[group_raw] = energy;
-        d.e_stats[group_raw * 2] += __popc(nonconv);
+        if (nonconv) d.e_stats[group_raw * 2] += __popc(nonconv);
         d.e_stats[group_raw * 2 + 1] = __popc(ypts);
     }
 }
