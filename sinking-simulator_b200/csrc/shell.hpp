@@ -146,8 +146,10 @@ constexpr int kShellBlock = 128;          // 16 elements per block
 // The step's per-element corner record in shared memory (floats): the corners' rest
 // differences to corner 0 (8 x 3), the bottom corners' directors (4 x 3), the
 // displacement differences to corner 0 (8 x 3), the co-rotated displacements (8 x 3)
-// the centre's Voigt transform T0 (4 columns x 6) and the factor of K_aa (28).
-constexpr int kGeoX = 0, kGeoD = 24, kGeoDd = 36, kGeoU = 60, kGeoT = 84, kGeoL = 108, kShellGeo = 136;
+// the centre's Voigt transform T0 (4 columns x 6), the factor of K_aa (28) and the
+// rotation (9, then whether the element has forms).
+constexpr int kGeoX = 0, kGeoD = 24, kGeoDd = 36, kGeoU = 60, kGeoT = 84, kGeoL = 108, kGeoQ = 136,
+              kShellGeo = 148;
 constexpr int kShellNodeBlock = 256;
 constexpr int kShellPunchBlock = 256;   // the inertial punch: one block
 constexpr int kShellFiberBlock = 128;

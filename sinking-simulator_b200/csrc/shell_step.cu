@@ -410,6 +410,81 @@ __device__ __noinline__ bool shell_tangent_factor(float n0, float n1, float n2, 
     return spd;
 }
 
+// The element's rotation from its corners' displacement differences dd (8 x 3):
+// H = (sum_a dN_a(0) (x) dd_a) J0^-1, R = I + Q.
+__device__ __forceinline__ void shell_rotation(const float (&dd)[24], const float (&j0)[9], float (&q)[9]) {
+    const float sx[8] = {-1, 1, 1, -1, -1, 1, 1, -1}, sy[8] = {-1, -1, 1, 1, -1, -1, 1, 1},
+                sz[8] = {-1, -1, -1, -1, 1, 1, 1, 1};
+    float jd[9];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+            const float v = dd[a * 3 + i];
+            a0 += sx[a] * v;
+            a1 += sy[a] * v;
+            a2 += sz[a] * v;
+        }
+        jd[i * 3] = 0.125f * a0;
+        jd[i * 3 + 1] = 0.125f * a1;
+        jd[i * 3 + 2] = 0.125f * a2;
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) q[i * 3 + j] = jd[i * 3] * j0[j] + jd[i * 3 + 1] * j0[3 + j] + jd[i * 3 + 2] * j0[6 + j];
+    // Higham iteration to convergence in FP32 (the CPU runs it to 1e-16 in double,
+    // solid_shell.cpp:473-487), at most six iterations.  The iteration converges
+    // quadratically: X = R (I + E) goes to R (I + E^2 / 2), and a step moves Q by
+    // about |E|, so after a step of size s the next would move it by about s^2 / 2.
+    // Stop once that is within an FP32 ulp of |Q| (s^2 <= 2.4e-7 |Q|), or once a
+    // step itself moved Q by no more than a few ulps (4.8e-7 |Q|).
+#pragma unroll 1
+    for (int it = 0; it < 6; ++it) {
+        float ipq[9], m[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) ipq[k] = q[k];
+        ipq[0] += 1.0f;
+        ipq[4] += 1.0f;
+        ipq[8] += 1.0f;
+        inv3f(ipq, m);
+        float mq[9];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) mq[i * 3 + j] = m[i * 3] * q[j] + m[i * 3 + 1] * q[3 + j] + m[i * 3 + 2] * q[6 + j];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) ipq[i * 3 + j] = 0.5f * (q[i * 3 + j] - mq[j * 3 + i]);
+        float step = 0.0f, size = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            step = fmaxf(step, fabsf(ipq[k] - q[k]));
+            size = fmaxf(size, fabsf(ipq[k]));
+            q[k] = ipq[k];
+        }
+        if (step <= 4.8e-7f * size || step * step <= 2.4e-7f * size) break;
+    }
+}
+
+// An element row: J0^-1 and the enhanced-mode scales; whether it has valid forms (it is
+// all zero otherwise).
+__device__ __forceinline__ bool shell_row(const float4* row, float (&j0)[9], float (&cm)[7]) {
+    const float4 r0 = row[0], r1 = row[1], r2 = row[2], r3 = row[3];
+    const float v[16] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
+    bool formed = false;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        j0[k] = v[k];
+        formed = formed || v[k] != 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < 7; ++k) cm[k] = v[9 + k];
+    return formed;
+}
+
 // Blocks per SM the register budget is sized for, chosen per launch.  With the
 // operators formed in the kernel the element pass is issue- and latency-bound.  A zone
 // that fills the GPU wants warps to hide latency, more than it minds spills: on the
@@ -551,83 +626,49 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
         }
         __syncwarp();
     }
-    float j0[9], cm[7];
-    {
-        const float4* row = d.elem + e * kShellElemQ;
-        if constexpr (PARK) {
-            cp_async_wait_one();  // the row's copies, by four of the element's lanes
-            __syncwarp();
-            row = row_park[threadIdx.x >> 3];
+    // ---- the element's rotation, and T0 of G's factored form (column j of G = gc_j T0[:,
+    // k_j], k = (0, 1, 2, 2, 2, 3, 3)), both the same for its eight lanes; T0 lies in the
+    // element's record in shared memory rather than in 24 registers of every lane ----
+    const auto element_part = [](const float (&j0)[9], float* record, float (&q)[9]) {
+        float dd[24], T0[24];
+        load_record<24>(record + kGeoDd, dd);
+        shell_rotation(dd, j0, q);
+        shell_t0(j0, T0);
+        float4* t4 = reinterpret_cast<float4*>(record + kGeoT);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) t4[k] = make_float4(T0[4 * k], T0[4 * k + 1], T0[4 * k + 2], T0[4 * k + 3]);
+    };
+    float cm[7], q[9];
+    bool formed;
+    if constexpr (PARK) {
+        // A wide zone is bound by issue slots: one lane an element does it, the block's
+        // sixteen elements side by side in half a warp, instead of each in eight lanes.
+        cp_async_wait_one();  // the rows' copies
+        __syncthreads();
+        if (threadIdx.x < kShellBlock / 8) {
+            float j0[9];
+            float* record = geo_park[threadIdx.x];
+            const bool any = shell_row(row_park[threadIdx.x], j0, cm);
+            element_part(j0, record, q);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) record[kGeoQ + k] = q[k];
+            record[kGeoQ + 9] = any ? 1.0f : 0.0f;
         }
-        const float4 r0 = row[0], r1 = row[1], r2 = row[2], r3 = row[3];
-        const float v[16] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w, r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
+        __syncthreads();
+        float qr[12];
+        load_record<12>(geo + kGeoQ, qr);
 #pragma unroll
-        for (int k = 0; k < 9; ++k) j0[k] = v[k];
+        for (int k = 0; k < 9; ++k) q[k] = qr[k];
+        formed = qr[9] != 0.0f;
+        const float4* row = row_park[threadIdx.x >> 3];
+        const float4 r2 = row[2], r3 = row[3];
+        const float v[7] = {r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
 #pragma unroll
-        for (int k = 0; k < 7; ++k) cm[k] = v[9 + k];
-    }
-    bool formed = false;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) formed = formed || j0[k] != 0.0f;
-    // ---- rotation: H = (sum_a dN_a(0) (x) dd_a) J0^-1, R = I + Q ----
-    float q[9];
-    {
-        float dd[24];
-        load_record<24>(geo + kGeoDd, dd);
-        const float sx[8] = {-1, 1, 1, -1, -1, 1, 1, -1}, sy[8] = {-1, -1, 1, 1, -1, -1, 1, 1},
-                    sz[8] = {-1, -1, -1, -1, 1, 1, 1, 1};
-        float jd[9];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
-#pragma unroll
-            for (int a = 0; a < 8; ++a) {
-                const float v = dd[a * 3 + i];
-                a0 += sx[a] * v;
-                a1 += sy[a] * v;
-                a2 += sz[a] * v;
-            }
-            jd[i * 3] = 0.125f * a0;
-            jd[i * 3 + 1] = 0.125f * a1;
-            jd[i * 3 + 2] = 0.125f * a2;
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) q[i * 3 + j] = jd[i * 3] * j0[j] + jd[i * 3 + 1] * j0[3 + j] + jd[i * 3 + 2] * j0[6 + j];
-        // Higham iteration to convergence in FP32 (the CPU runs it to 1e-16 in double,
-        // solid_shell.cpp:473-487), at most six iterations.  The iteration converges
-        // quadratically: X = R (I + E) goes to R (I + E^2 / 2), and a step moves Q by
-        // about |E|, so after a step of size s the next would move it by about s^2 / 2.
-        // Stop once that is within an FP32 ulp of |Q| (s^2 <= 2.4e-7 |Q|), or once a
-        // step itself moved Q by no more than a few ulps (4.8e-7 |Q|).
-#pragma unroll 1
-        for (int it = 0; it < 6; ++it) {
-            float ipq[9], m[9];
-#pragma unroll
-            for (int k = 0; k < 9; ++k) ipq[k] = q[k];
-            ipq[0] += 1.0f;
-            ipq[4] += 1.0f;
-            ipq[8] += 1.0f;
-            inv3f(ipq, m);
-            float mq[9];
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = 0; j < 3; ++j) mq[i * 3 + j] = m[i * 3] * q[j] + m[i * 3 + 1] * q[3 + j] + m[i * 3 + 2] * q[6 + j];
-#pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = 0; j < 3; ++j) ipq[i * 3 + j] = 0.5f * (q[i * 3 + j] - mq[j * 3 + i]);
-            float step = 0.0f, size = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 9; ++k) {
-                step = fmaxf(step, fabsf(ipq[k] - q[k]));
-                size = fmaxf(size, fabsf(ipq[k]));
-                q[k] = ipq[k];
-            }
-            if (step <= 4.8e-7f * size || step * step <= 2.4e-7f * size) break;
-        }
+        for (int k = 0; k < 7; ++k) cm[k] = v[k];
+    } else {
+        float j0[9];
+        formed = shell_row(d.elem + e * kShellElemQ, j0, cm);
+        element_part(j0, geo, q);
     }
     // ---- co-rotated relative displacement u'_a = Q^T dX_a + dd_a + Q^T dd_a, lane a's
     // corner formed by lane a and parked beside the others ----
@@ -641,11 +682,14 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
         __syncwarp();
     }
 
-    // the rotation waits in shared memory through the Newton iterations (each lane its
-    // own copy: no synchronisation), freeing nine registers there
-    __shared__ float q_park[9][kShellBlock];
+    // the rotation waits in shared memory through the Newton iterations, freeing nine
+    // registers there
+    if constexpr (!PARK) {
+        if (gp == 0) {
 #pragma unroll
-    for (int k = 0; k < 9; ++k) q_park[k][threadIdx.x] = q[k];
+            for (int k = 0; k < 9; ++k) geo[kGeoQ + k] = q[k];
+        }
+    }
     // ---- the point's operators, formed from the rest geometry ----
     const ShellLanePoint P = shell_lane_point(gp);
     float w, eps_u[6];
@@ -666,18 +710,7 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
         load_record<24>(geo + kGeoU, u);
         shell_strain(dX, D, u, P, gx, gy, Ainv, eps_u);
     }
-    // G factored: column j = gc_j T0[:, k_j], k = (0, 1, 2, 2, 2, 3, 3)
-    // T0 is the element's, the same in its eight lanes: one copy in the element's record
-    // in shared memory rather than 24 registers in every lane through the Newton loop
     float gc[7];
-    {
-        float T0[24];
-        shell_t0(j0, T0);
-        float4* t4 = reinterpret_cast<float4*>(geo + kGeoT);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) t4[k] = make_float4(T0[4 * k], T0[4 * k + 1], T0[4 * k + 2], T0[4 * k + 3]);
-        __syncwarp();
-    }
     const float* T = geo + kGeoT;
     shell_enhanced_scales(cm, w, P, gc);
     // element volume and the energy scale sigma_y V
@@ -1150,7 +1183,7 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
         float* out = d.slots + (size_t)slot * 3;
         float qr[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) qr[k] = q_park[k][threadIdx.x];
+        for (int k = 0; k < 9; ++k) qr[k] = geo[kGeoQ + k];
 #pragma unroll
         for (int i = 0; i < 3; ++i) out[i] = -(f[i] + (qr[i * 3] * f[0] + qr[i * 3 + 1] * f[1] + qr[i * 3 + 2] * f[2]));
     }
