@@ -119,7 +119,7 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
     s->mode = mode;
     s->nodes = N;
     s->tets = T;
-    s->eblocks = fs::blocks_for((long long)T, mode == FEMSTEP_TET_J2_F64 ? fs::kTet64Block : fs::kBlock);
+    s->eblocks = fs::blocks_for((long long)T, mode == FEMSTEP_TET_J2_F64 ? fs::kTet64Block : fs::kTetF32Block);
     s->nblocks = fs::blocks_for((long long)N, fs::kTetNodeBlock);
     int rc = check(s, cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "stream");
     if (rc == FEMSTEP_OK) rc = check(s, cudaEventCreate(&s->ev0), "event");
@@ -297,7 +297,7 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
     s->mode = mode;
     s->nodes = N;
     s->tets = T;
-    s->eblocks = fs::blocks_for((long long)T, mode == FEMSTEP_TET_J2_F64 ? fs::kTet64Block : fs::kBlock);
+    s->eblocks = fs::blocks_for((long long)T, mode == FEMSTEP_TET_J2_F64 ? fs::kTet64Block : fs::kTetF32Block);
     s->nblocks = fs::blocks_for((long long)N, fs::kTetNodeBlock);
     int rc = check(s, cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking), "stream");
     if (rc == FEMSTEP_OK) rc = check(s, cudaEventCreate(&s->ev0), "event");

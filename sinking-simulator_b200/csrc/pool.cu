@@ -42,7 +42,7 @@ __device__ __forceinline__ void element_tile(const PoolDevice& d, int tile, int 
     if (live && t < tl.end) tet_element_f32<true, CG>(element_refs(d), t, m.mat, diss, energy);
     block_sum2(diss, energy, scratch);  // valid in thread 0
     if (live && threadIdx.x == 0) {
-        d.e_diss[tl.part] += diss;
+        if (diss != 0.0) d.e_diss[tl.part] += diss;  // else the sum stands, unread
         d.e_strain[tl.part] = energy;
     }
 }
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(B, MINB) pool_elements_ring(PoolDevice d, int 
         }
         block_sum2(diss, energy, scratch);  // valid in thread 0; also the closing barrier
         if (threadIdx.x == 0 && live && ok) {
-            d.e_diss[tl.part] += diss;
+            if (diss != 0.0) d.e_diss[tl.part] += diss;  // else the sum stands, unread
             d.e_strain[tl.part] = energy;
         }
         if (next >= d.n_etiles) break;

@@ -120,7 +120,8 @@ cudaError_t build_runs_device(const uint32_t* offset, const uint32_t* entry, lon
 // Threads per block of the single-mesh node kernels: few, so that a small mesh's nodes
 // spread over the SMs.
 constexpr int kTetNodeBlock = 128;
-constexpr int kTet64Block = 128;  // threads per block of the FP64 element kernel
+constexpr int kTet64Block = 128;   // threads per block of the FP64 element kernel,
+constexpr int kTetF32Block = 128;  // and of the FP32 J2 modes'
 constexpr int kElementPart = 1, kNodePart = 2, kWholeStep = 3;
 void launch_ref32_step(const TetDevice<float>& d, const TetParams& p, cudaStream_t stream,
                        int parts = kWholeStep);

@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d
     }
     block_sum2(diss, energy, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
-        d.e_diss[blockIdx.x] += diss;
+        if (diss != 0.0) d.e_diss[blockIdx.x] += diss;  // else the sum stands, unread
         d.e_strain[blockIdx.x] = energy;
     }
 }

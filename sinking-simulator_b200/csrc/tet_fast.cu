@@ -24,9 +24,9 @@ __device__ __forceinline__ TetElementRefs refs(const TetDevice<float>& d) {
                           d.tets};
 }
 
-// 1024 / kBlock blocks per SM: 64 registers, 32 resident warps per SM
+// 1024 / kTetF32Block blocks per SM: 64 registers, 32 resident warps per SM
 template <bool KAHAN>
-__global__ void __launch_bounds__(kBlock, 1024 / kBlock) f32_forces(TetDevice<float> d, J2f m, int wave) {
+__global__ void __launch_bounds__(kTetF32Block, 1024 / kTetF32Block) f32_forces(TetDevice<float> d, J2f m, int wave) {
     __shared__ double scratch[64];
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     {
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kBlock, 1024 / kBlock) f32_forces(TetDevice<fl
     if (t < d.tets) tet_element_f32<KAHAN, false, LoadedRows>(r, rows, t, m, diss, energy);
     block_sum2(diss, energy, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
-        d.e_diss[blockIdx.x] += diss;
+        if (diss != 0.0) d.e_diss[blockIdx.x] += diss;  // else the sum stands, unread
         d.e_strain[blockIdx.x] = energy;
     }
 }
@@ -94,16 +94,16 @@ __global__ void __launch_bounds__(kTetNodeBlock) f32_nodes(TetDevice<float> d, f
 
 void launch_f32_step(const TetDevice<float>& d, const TetParams& p, bool compensated, cudaStream_t stream,
                      int parts) {
-    const int eb = blocks_for(d.tets, kBlock), nb = blocks_for(d.nodes, kTetNodeBlock);
+    const int eb = blocks_for(d.tets, kTetF32Block), nb = blocks_for(d.nodes, kTetNodeBlock);
     const J2f m = make_j2f(p.mu, p.bulk, p.yield, p.hardening);
-    const int wave = sm_count() * (1024 / kBlock);
+    const int wave = sm_count() * (1024 / kTetF32Block);
     if (compensated) {
-        if (parts & kElementPart) launch_pdl(f32_forces<true>, eb, kBlock, 0, stream, d, m, wave);
+        if (parts & kElementPart) launch_pdl(f32_forces<true>, eb, kTetF32Block, 0, stream, d, m, wave);
         if (parts & kNodePart)
             launch_pdl(f32_nodes<true>, nb, kTetNodeBlock, 0, stream, d, (float)p.dt, (float)p.gravity, (float)p.damping,
                        p.ramp);
     } else {
-        if (parts & kElementPart) launch_pdl(f32_forces<false>, eb, kBlock, 0, stream, d, m, wave);
+        if (parts & kElementPart) launch_pdl(f32_forces<false>, eb, kTetF32Block, 0, stream, d, m, wave);
         if (parts & kNodePart)
             launch_pdl(f32_nodes<false>, nb, kTetNodeBlock, 0, stream, d, (float)p.dt, (float)p.gravity,
                        (float)p.damping, p.ramp);
