@@ -7,6 +7,7 @@
 // no device is a skip, not an abort).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -105,6 +106,32 @@ void launch_step(femstep_tet* s, const TetParams& q, int parts = fs::kWholeStep)
 }
 
 constexpr int kGraphSteps = 32;
+
+// A run of at least kClusterSteps steps of a mesh that fits one cluster of blocks is one
+// launch per kClusterChunk steps.  Shorter runs keep two launches a step, which is what
+// femstep_tet_launches reports for them.
+constexpr int kClusterSteps = 128, kClusterChunk = 1024;
+
+// Up to `substeps` steps that way; how many were queued.
+int run_cluster(femstep_tet* s, int substeps, const TetParams& q) {
+    const size_t most = s->mode == FEMSTEP_TET_J2_F64 ? fs::kCluster64Most : fs::kClusterMost;
+    if (substeps < kClusterSteps || s->tets > most || s->nodes > most) return 0;
+    int queued = 0;
+    while (queued < substeps) {
+        const int n = std::min(substeps - queued, kClusterChunk);
+        bool ok = false;
+        switch (s->mode) {
+            case FEMSTEP_TET_REF32: ok = fs::launch_ref32_cluster(s->d32, q, n, s->stream); break;
+            case FEMSTEP_TET_J2_F32: ok = fs::launch_f32_cluster(s->d32, q, false, n, s->stream); break;
+            case FEMSTEP_TET_J2_F32K: ok = fs::launch_f32_cluster(s->d32, q, true, n, s->stream); break;
+            default: ok = fs::launch_f64_cluster(s->d64, q, n, s->stream); break;
+        }
+        if (!ok) break;
+        queued += n;
+        ++s->launches;
+    }
+    return queued;
+}
 
 // femstep_tet_create for the J2 modes when the caller gives no adjacency (the mesh is
 // already checked): everything from the caller's node positions and node ids on the
@@ -427,7 +454,7 @@ int femstep_tet_run(femstep_tet* s, int substeps, const femstep_tet_params* para
     if (rc) return rc;
     // Whole chunks replay one captured graph of kGraphSteps steps; the rest launch
     // directly.  The graph bakes the parameters in, so it is rebuilt when they change.
-    int left = substeps;
+    int left = substeps - run_cluster(s, substeps, q);
     if (left >= kGraphSteps) {
         if (!s->graph || std::memcmp(&s->graph_params, &q, sizeof(q)) != 0) {
             if (s->graph) cudaGraphExecDestroy(s->graph);

@@ -129,6 +129,13 @@ void launch_f64_step(const TetDevice<double>& d, const TetParams& p, cudaStream_
                      int parts = kWholeStep);
 void launch_f32_step(const TetDevice<float>& d, const TetParams& p, bool compensated,
                      cudaStream_t stream, int parts = kWholeStep);
+// `steps` whole steps of a mesh of at most kClusterMost tets and nodes in one launch
+// (kCluster64Most for FP64); false, with nothing queued, where the device does not take it.
+// The state it leaves is the steps' to the bit.
+constexpr int kCluster64Most = 4096;
+bool launch_ref32_cluster(const TetDevice<float>& d, const TetParams& p, int steps, cudaStream_t stream);
+bool launch_f64_cluster(const TetDevice<double>& d, const TetParams& p, int steps, cudaStream_t stream);
+bool launch_f32_cluster(const TetDevice<float>& d, const TetParams& p, bool compensated, int steps, cudaStream_t stream);
 // FP64 element eigenvalue bound: omega^2 per tet, reduced to the maximum on device.
 void launch_tet_omega2(long long tets, const double* rest_inv, double E, double nu, double rho,
                        double* per_block_max, int blocks, cudaStream_t stream);

@@ -17,6 +17,8 @@
 // Memory-bound kernels (algorithmic bytes: ~240 B per update for REF32, ~435 B for
 // F64): one thread per tet / per node, SoA element arrays so each warp load is one
 // contiguous 128 B line, node-major force slots so each node's gather is contiguous.
+#include <algorithm>
+
 #include "common.cuh"
 #include "omega.cuh"
 #include "tet.hpp"
@@ -140,13 +142,26 @@ struct PolarPark {
     int count[2];
 };
 
+// The 128 threads of a park meet: a group of a larger block (GROUP), or the whole block --
+// with the one barrier, since a block that names barriers by number reserves all sixteen,
+// and an SM has enough of them for four such blocks only.
+template <bool GROUP>
+__device__ __forceinline__ void park_barrier() {
+    if (GROUP)
+        asm volatile("bar.sync %0, 128;" ::"r"((int)threadIdx.x >> 7) : "memory");
+    else
+        __syncthreads();
+}
+
+template <bool GROUP>
 __device__ __forceinline__ M3<double> polar_block(M3<double> r, bool live, PolarPark& park) {
+    static_assert(kTet64Block == 128, "a park serves one group of 128 threads");
     constexpr int kFirst = 6, kSnapshot = 10, kSecond = 16, kLast = 64;
     static_assert((kLast - kSecond) % (kSecond - kSnapshot) == 0, "whole periods remain");
     static_assert(kFirst % 2 == 0 && kSnapshot % 2 == 0 && kSecond % 2 == 0 && kLast % 2 == 0, "steps go in pairs");
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x & 127;
     if (tid < 2) park.count[tid] = 0;
-    __syncthreads();
+    park_barrier<GROUP>();
     bool done = !live || polar_step(r) || polar_step(r);
 #pragma unroll 1
     for (int it = 2; it < kFirst && !done; it += 2) done = polar_pair(r);
@@ -155,7 +170,7 @@ __device__ __forceinline__ M3<double> polar_block(M3<double> r, bool live, Polar
     if (!done) park.list[0][atomicAdd(&park.count[0], 1)] = (uint16_t)tid;
 #pragma unroll 1
     for (int round = 0; round < 2; ++round) {
-        __syncthreads();
+        park_barrier<GROUP>();
         const int n = park.count[round];
         if (n == 0) break;  // the same for the whole block
         if (tid < n) {
@@ -184,37 +199,24 @@ __device__ __forceinline__ M3<double> polar_block(M3<double> r, bool live, Polar
             for (int k = 0; k < 9; ++k) park.r[k][at] = x.m[k];
         }
     }
-    __syncthreads();
+    park_barrier<GROUP>();
 #pragma unroll
     for (int k = 0; k < 9; ++k) r.m[k] = park.r[k][tid];
     return r;
 }
 
 // ---------------------------------------------------------------------------------
-// REF32: fem::tetForces, written to the node-major slots.
-__global__ void __launch_bounds__(kBlock) ref32_forces(TetDevice<float> d, float lambda, float mu) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long tr = t < d.tets ? t : d.tets - 1;
-    const uint4 idx = d.index[tr], sl = d.slot[tr];
-    M3<float> dm_inv;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) dm_inv.m[k] = d.rest_inv[(size_t)k * d.tets + tr];
-    const float scale = -d.rest_vol[tr];
-    pdl_wait();
-    pdl_next();
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const long long s = d.counter[0];
-        d.counter[1] = s;
-        d.counter[0] = s + 1;
-    }
-    if (t >= d.tets) return;
+// REF32: fem::tetForces (fem.cpp:73-117), the corner forces written to their slots.  CG: the
+// positions were written by other SMs in this launch.
+template <bool CG>
+__device__ __forceinline__ void ref32_element(const float* p, const uint4& idx, const uint4& sl, const M3<float>& dm_inv,
+                                              float scale, float lambda, float mu, float* slot_array) {
     const unsigned nid[4] = {idx.x, idx.y, idx.z, idx.w};
-    const float* p = d.position;
     M3<float> ds;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int a = 0; a < 3; ++a) ds(a, c) = p[(size_t)nid[c + 1] * 3 + a] - p[(size_t)nid[0] * 3 + a];
+        for (int a = 0; a < 3; ++a) ds(a, c) = ldg_coherent<CG>(p + (size_t)nid[c + 1] * 3 + a) - ldg_coherent<CG>(p + (size_t)nid[0] * 3 + a);
     const M3<float> f = mul(ds, dm_inv);
     const M3<float> r = polar_fixed4(f);
     const M3<float> s = mul(transpose(r), f);
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(kBlock) ref32_forces(TetDevice<float> d, float
     const M3<float> h = mul(mul(r, stress), transpose(dm_inv));
     const unsigned sid[4] = {sl.x, sl.y, sl.z, sl.w};
     float f0[3] = {0.0f, 0.0f, 0.0f};
-    float4* slots = reinterpret_cast<float4*>(d.slots);
+    float4* slots = reinterpret_cast<float4*>(slot_array);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         float v[3];
@@ -246,6 +248,37 @@ __global__ void __launch_bounds__(kBlock) ref32_forces(TetDevice<float> d, float
         slots[sid[c + 1]] = make_float4(v[0], v[1], v[2], 0.0f);
     }
     slots[sid[0]] = make_float4(f0[0], f0[1], f0[2], 0.0f);
+}
+
+// REF32: a free node of fem::stepCpu's loop (fem.cpp:196-214).
+__device__ __forceinline__ void ref32_node(float m, const float (&force)[3], float dt, float damping, float* vel, float* pos) {
+    const float inv_mass = 1.0f / m;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float v = vel[k] + force[k] * inv_mass * dt;
+        v *= damping;
+        vel[k] = v;
+        pos[k] += v * dt;
+    }
+}
+
+__global__ void __launch_bounds__(kBlock) ref32_forces(TetDevice<float> d, float lambda, float mu) {
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long tr = t < d.tets ? t : d.tets - 1;
+    const uint4 idx = d.index[tr], sl = d.slot[tr];
+    M3<float> dm_inv;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) dm_inv.m[k] = d.rest_inv[(size_t)k * d.tets + tr];
+    const float scale = -d.rest_vol[tr];
+    pdl_wait();
+    pdl_next();
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        const long long s = d.counter[0];
+        d.counter[1] = s;
+        d.counter[0] = s + 1;
+    }
+    if (t >= d.tets) return;
+    ref32_element<false>(d.position, idx, sl, dm_inv, scale, lambda, mu, d.slots);
 }
 
 // REF32: fem::stepCpu's node loop (fem.cpp:196-214).
@@ -275,14 +308,57 @@ __global__ void __launch_bounds__(kTetNodeBlock) ref32_nodes(TetDevice<float> d,
             force[1] += f.y;
             force[2] += f.z;
         });
-    const float inv_mass = 1.0f / m;
-    float* pos = d.position + (size_t)n * 3;
+    ref32_node(m, force, dt, damping, vel, d.position + (size_t)n * 3);
+}
+
+// `steps` steps of a small mesh in one cluster (common.cuh), with the two kernels' arithmetic.
+__global__ void __launch_bounds__(512) ref32_cluster(TetDevice<float> d, float lambda, float mu, float dt, float gravity,
+                                                     float damping, int steps) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, ni = cluster_node_group() * 128 + (threadIdx.x & 127);
+    const bool tet = i < d.tets, node = ni < d.nodes;
+    const long long t = tet ? i : 0;
+    const uint4 idx = d.index[t], sl = d.slot[t];
+    M3<float> dm_inv;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) dm_inv.m[k] = d.rest_inv[(size_t)k * d.tets + t];
+    const float scale = -d.rest_vol[t];
+    const int n = node ? ni : 0;
+    const SlotRun run = slot_run(d.run[n]);
+    const float m = d.mass[n];
+    const bool held = !node || d.fixed[n] != 0;
+    const float4* slots = reinterpret_cast<const float4*>(d.slots);
+    float vel[3], pos[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        float v = vel[k] + force[k] * inv_mass * dt;
-        v *= damping;
-        vel[k] = v;
-        pos[k] += v * dt;
+        vel[k] = held ? 0.0f : d.velocity[(size_t)n * 3 + k];
+        pos[k] = d.position[(size_t)n * 3 + k];
+    }
+    const long long first = d.counter[0];
+    for (int s = 0; s < steps; ++s) {
+        if (tet) ref32_element<true>(d.position, idx, sl, dm_inv, scale, lambda, mu, d.slots);
+        cluster_barrier();
+        if (!held) {
+            float force[3] = {0.0f, 0.0f, -gravity * m};
+            for_run<12>(
+                run, [&](uint32_t k) { return __ldcg(slots + k); },
+                [&](const float4& f) {
+                    force[0] += f.x;
+                    force[1] += f.y;
+                    force[2] += f.z;
+                });
+            ref32_node(m, force, dt, damping, vel, pos);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) d.position[(size_t)n * 3 + k] = pos[k];
+        }
+        cluster_barrier();
+    }
+    if (node) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) d.velocity[(size_t)n * 3 + k] = vel[k];
+    }
+    if (i == 0) {
+        d.counter[0] = first + steps;
+        d.counter[1] = first + steps - 1;
     }
 }
 
@@ -377,51 +453,42 @@ __device__ __forceinline__ J2Out j2_return_f64(const double strain[6], double ps
     return out;
 }
 
-__global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d, TetParams p) {
-    __shared__ double scratch[64];
-    __shared__ PolarPark park;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = t < d.tets;
-    uint4 idx = make_uint4(0, 0, 0, 0);
-    if (live) {
-        idx = d.index[t];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) cp_async8(&park.rows[k][threadIdx.x], d.rest_inv + (size_t)k * d.tets + t);
-        cp_async_commit();
-        cp_async8(&park.rows[9][threadIdx.x], d.rest_vol + t);
-    }
-    pdl_wait();
-    pdl_next();
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const long long s = d.counter[0];
-        d.counter[1] = s;
-        d.counter[0] = s + 1;
-    }
-    double diss = 0.0, energy = 0.0;
+// One tet of the FP64 step (every thread of its 128-thread group calls it, `live` or not):
+// its Dm^-1 and volume in the park's rows (their copies under way), its plastic state
+// copied there too; corner forces to their slots.  CG: in a cluster run, where other SMs
+// wrote the positions in this launch and the rows stay in the park from step to step.
+template <bool CG>
+__device__ __forceinline__ void f64_element(const TetDevice<double>& d, const TetParams& p, PolarPark& park, long long t,
+                                            bool live, const uint4& idx, double& diss, double& energy) {
+    const int tid = threadIdx.x & 127;
+    diss = energy = 0.0;
     M3<double> f;
     if (live) {
         const unsigned nid[4] = {idx.x, idx.y, idx.z, idx.w};
         const double* x = d.position;
+        const auto load = [](const double* at) { return CG ? __ldcg(at) : *at; };
         M3<double> ds, dm_inv;
+        if (!CG) {
 #pragma unroll
-        for (int i = 0; i < 7; ++i) cp_async8(&park.rows[10 + i][threadIdx.x], d.plastic + (size_t)i * d.tets + t);
-        cp_async_commit();
+            for (int i = 0; i < 7; ++i) cp_async8(&park.rows[10 + i][tid], d.plastic + (size_t)i * d.tets + t);
+            cp_async_commit();
+        }
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int a = 0; a < 3; ++a) ds(a, c) = x[(size_t)nid[c + 1] * 3 + a] - x[(size_t)nid[0] * 3 + a];
-        cp_async_wait_one();  // a thread reads back only what it copied: no barrier
+            for (int a = 0; a < 3; ++a) ds(a, c) = load(x + (size_t)nid[c + 1] * 3 + a) - load(x + (size_t)nid[0] * 3 + a);
+        if (!CG) cp_async_wait_one();  // a thread reads back only what it copied: no barrier
 #pragma unroll
-        for (int k = 0; k < 9; ++k) dm_inv.m[k] = park.rows[k][threadIdx.x];
+        for (int k = 0; k < 9; ++k) dm_inv.m[k] = park.rows[k][tid];
         f = mul(ds, dm_inv);
 #pragma unroll
-        for (int k = 0; k < 9; ++k) park.f[k][threadIdx.x] = f.m[k];
+        for (int k = 0; k < 9; ++k) park.f[k][tid] = f.m[k];
     }
-    const M3<double> r = polar_block(f, live, park);
+    const M3<double> r = polar_block<CG>(f, live, park);
     if (live) {
-        cp_async_wait_all();
+        if (!CG) cp_async_wait_all();
 #pragma unroll
-        for (int k = 0; k < 9; ++k) f.m[k] = park.f[k][threadIdx.x];
+        for (int k = 0; k < 9; ++k) f.m[k] = park.f[k][tid];
         const M3<double> sm = mul(transpose(r), f);
         double strain[6];
         strain[0] = 0.5 * (sm(0, 0) + sm(0, 0)) - 1.0;
@@ -432,14 +499,17 @@ __global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d
         strain[5] = 2.0 * (0.5 * (sm(2, 0) + sm(0, 2)));
         double ps[7];
 #pragma unroll
-        for (int i = 0; i < 7; ++i) ps[i] = park.rows[10 + i][threadIdx.x];
+        for (int i = 0; i < 7; ++i) ps[i] = park.rows[10 + i][tid];
         double sv[6];
         const J2Out j = j2_return_f64(strain, ps, p.mu, p.bulk, p.yield, p.hardening, sv);
         if (j.yielded) {
 #pragma unroll
-            for (int i = 0; i < 7; ++i) d.plastic[(size_t)i * d.tets + t] = ps[i];
+            for (int i = 0; i < 7; ++i) {
+                d.plastic[(size_t)i * d.tets + t] = ps[i];
+                if (CG) park.rows[10 + i][tid] = ps[i];
+            }
         }
-        const double vol = park.rows[9][threadIdx.x];
+        const double vol = park.rows[9][tid];
         diss = vol * j.dissipation;
         // 1/2 sigma : C^-1 : sigma from the deviator and the trace, by the reciprocals
         const double tr = sv[0] + sv[1] + sv[2], pressure = tr * (1.0 / 3.0);
@@ -449,7 +519,7 @@ __global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d
 
         M3<double> dm_inv;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) dm_inv.m[k] = park.rows[k][threadIdx.x];
+        for (int k = 0; k < 9; ++k) dm_inv.m[k] = park.rows[k][tid];
 
         M3<double> stress;
         stress(0, 0) = sv[0];
@@ -479,10 +549,49 @@ __global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d
         xy[sid[0]] = make_double2(f0[0], f0[1]);
         z[sid[0]] = f0[2];
     }
+}
+
+__global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d, TetParams p) {
+    __shared__ double scratch[64];
+    __shared__ PolarPark park;
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = t < d.tets;
+    uint4 idx = make_uint4(0, 0, 0, 0);
+    if (live) {
+        idx = d.index[t];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) cp_async8(&park.rows[k][threadIdx.x], d.rest_inv + (size_t)k * d.tets + t);
+        cp_async_commit();
+        cp_async8(&park.rows[9][threadIdx.x], d.rest_vol + t);
+    }
+    pdl_wait();
+    pdl_next();
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+        const long long s = d.counter[0];
+        d.counter[1] = s;
+        d.counter[0] = s + 1;
+    }
+    double diss, energy;
+    f64_element<false>(d, p, park, t, live, idx, diss, energy);
     block_sum2(diss, energy, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
         if (diss != 0.0) d.e_diss[blockIdx.x] += diss;  // else the sum stands, unread
         d.e_strain[blockIdx.x] = energy;
+    }
+}
+
+// A free node's update from the force on it (its external part included), and the step's
+// external work and kinetic energy.
+__device__ __forceinline__ void f64_node(const TetParams& p, double m, double inv_mass, const double (&force)[3],
+                                         const double (&ext)[3], double* vel, double* pos, double& work, double& kin) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        double v = vel[k] + force[k] * inv_mass * p.dt;
+        v *= p.damping;
+        vel[k] = v;
+        pos[k] += v * p.dt;
+        work += ext[k] * v * p.dt;
+        kin += 0.5 * m * v * v;
     }
 }
 
@@ -523,17 +632,7 @@ __global__ void __launch_bounds__(kTetNodeBlock) f64_nodes(TetDevice<double> d, 
             }
 #pragma unroll
             for (int k = 0; k < 3; ++k) force[k] += ext[k];
-            const double inv_mass = 1.0 / m;
-            double* pos = d.position + (size_t)n * 3;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                double v = vel[k] + force[k] * inv_mass * p.dt;
-                v *= p.damping;
-                vel[k] = v;
-                pos[k] += v * p.dt;
-                work += ext[k] * v * p.dt;
-                kin += 0.5 * m * v * v;
-            }
+            f64_node(p, m, 1.0 / m, force, ext, vel, d.position + (size_t)n * 3, work, kin);
             gwork = -p.gravity * m * vel[2] * p.dt;
         }
     }
@@ -545,6 +644,106 @@ __global__ void __launch_bounds__(kTetNodeBlock) f64_nodes(TetDevice<double> d, 
     if (p.gravity != 0.0) {
         gwork = block_sum(gwork, scratch);
         if (threadIdx.x == 0) d.n_grav[blockIdx.x] += gwork;
+    }
+}
+
+// `steps` steps of a small mesh in one cluster (common.cuh), with the two kernels'
+// arithmetic and sums.  A group of 128 threads has its own park; Dm^-1, volumes and the
+// plastic state stay there for the run.
+__global__ void __launch_bounds__(kCluster64Most / kClusterBlocks) f64_cluster(TetDevice<double> d, TetParams p, int steps) {
+    extern __shared__ __align__(16) unsigned char parks[];
+    __shared__ GroupSums esum, nsum, gsum;
+    PolarPark& park = reinterpret_cast<PolarPark*>(parks)[threadIdx.x >> 7];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, group = i >> 7, tid = threadIdx.x & 127;
+    const int node_group = cluster_node_group(), ni = node_group * 128 + tid;
+    const bool leader = tid == 0, tet = i < d.tets, node = ni < d.nodes;
+    const long long t = tet ? i : 0;
+    const uint4 idx = d.index[t];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) park.rows[k][tid] = d.rest_inv[(size_t)k * d.tets + t];
+    park.rows[9][tid] = d.rest_vol[t];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) park.rows[10 + k][tid] = d.plastic[(size_t)k * d.tets + t];
+    const int n = node ? ni : 0;
+    const SlotRun run = slot_run(d.run[n]);
+    const bool held = !node || d.fixed[n] != 0;
+    const double m = d.mass[n], inv_mass = 1.0 / m;
+    double load[3] = {0.0, 0.0, 0.0}, vel[3], pos[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (d.ext) load[k] = d.ext[(size_t)n * 3 + k];
+        vel[k] = held ? 0.0 : d.velocity[(size_t)n * 3 + k];
+        pos[k] = d.position[(size_t)n * 3 + k];
+    }
+    const double2* xy = reinterpret_cast<const double2*>(d.slots);
+    const double* z = d.slots + 2 * d.slot_count;
+    const bool eg = leader && (long long)group * 128 < d.tets, ng = leader && (long long)node_group * 128 < d.nodes;
+    double dissipated = eg ? d.e_diss[group] : 0.0, strain = 0.0;
+    double worked = ng ? d.n_work[node_group] : 0.0, kinetic = 0.0, fallen = ng ? d.n_grav[node_group] : 0.0;
+    const long long first = d.counter[0];
+    for (int s = 0; s < steps; ++s) {
+        double diss, energy;
+        f64_element<true>(d, p, park, t, tet, idx, diss, energy);
+        esum.put(diss, energy);
+        cluster_barrier();
+        if (leader) {
+            const double2 e = esum.get();
+            if (e.x != 0.0) dissipated += e.x;
+            strain = e.y;
+        }
+        double work = 0.0, kin = 0.0, gwork = 0.0;
+        if (!held) {
+            const double lf = ramp_factor(first + s, p.ramp);
+            double force[3] = {0.0, 0.0, -p.gravity * m};
+            for_run<8>(
+                run,
+                [&](uint32_t k) {
+                    const double2 f = __ldcg(xy + k);
+                    return make_double3(f.x, f.y, __ldcg(z + k));
+                },
+                [&](const double3& f) {
+                    force[0] += f.x;
+                    force[1] += f.y;
+                    force[2] += f.z;
+                });
+            double ext[3] = {0.0, 0.0, 0.0};
+            if (d.ext) {
+#pragma unroll
+                for (int k = 0; k < 3; ++k) ext[k] = lf * load[k];
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k) force[k] += ext[k];
+            f64_node(p, m, inv_mass, force, ext, vel, pos, work, kin);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) d.position[(size_t)n * 3 + k] = pos[k];
+            gwork = -p.gravity * m * vel[2] * p.dt;
+        }
+        nsum.put(work, kin);
+        if (p.gravity != 0.0) gsum.put(gwork, 0.0);
+        cluster_barrier();
+        if (leader) {
+            const double2 w = nsum.get();
+            worked += w.x;
+            kinetic = w.y;
+            if (p.gravity != 0.0) fallen += gsum.get().x;
+        }
+    }
+    if (node) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) d.velocity[(size_t)n * 3 + k] = vel[k];
+    }
+    if (eg) {
+        d.e_diss[group] = dissipated;
+        d.e_strain[group] = strain;
+    }
+    if (ng) {
+        d.n_work[node_group] = worked;
+        d.n_kin[node_group] = kinetic;
+        if (p.gravity != 0.0) d.n_grav[node_group] = fallen;
+    }
+    if (i == 0) {
+        d.counter[0] = first + steps;
+        d.counter[1] = first + steps - 1;
     }
 }
 
@@ -698,6 +897,19 @@ void launch_ref32_step(const TetDevice<float>& d, const TetParams& p, cudaStream
     if (parts & kNodePart)
         launch_pdl(ref32_nodes, blocks_for(d.nodes, kTetNodeBlock), kTetNodeBlock, 0, stream, d, (float)p.dt,
                    (float)p.gravity, (float)p.damping);
+}
+
+bool launch_ref32_cluster(const TetDevice<float>& d, const TetParams& p, int steps, cudaStream_t stream) {
+    int blocks, threads;
+    cluster_shape(std::max(d.tets, d.nodes), blocks, threads);
+    return launch_cluster(ref32_cluster, blocks, threads, 0, stream, d, (float)p.lambda, (float)p.mu, (float)p.dt,
+                          (float)p.gravity, (float)p.damping, steps);
+}
+
+bool launch_f64_cluster(const TetDevice<double>& d, const TetParams& p, int steps, cudaStream_t stream) {
+    int blocks, threads;
+    cluster_shape(std::max(d.tets, d.nodes), blocks, threads);
+    return launch_cluster(f64_cluster, blocks, threads, sizeof(PolarPark) * (threads / 128), stream, d, p, steps);
 }
 
 void launch_f64_step(const TetDevice<double>& d, const TetParams& p, cudaStream_t stream, int parts) {

@@ -73,20 +73,6 @@ __device__ __forceinline__ M3<float> inverse_fma(const M3<float>& a, float tiny)
     return r;
 }
 
-// A global load that bypasses L1 when CG: needed where another SM wrote the data
-// earlier in the same (persistent) launch.
-template <bool CG>
-__device__ __forceinline__ float ldg_coherent(const float* p) {
-    if (CG) return __ldcg(p);
-    return *p;
-}
-
-template <bool CG>
-__device__ __forceinline__ float4 ldg_coherent4(const float4* p) {
-    if (CG) return __ldcg(p);
-    return *p;
-}
-
 struct TetElementRefs {
     const uint4* index;     // [stride] node ids
     const uint4* slot;      // [stride] node-major slot of each corner
@@ -415,6 +401,28 @@ struct TetNodeRefs {
     float4* disp_c;          // compensated variant
 };
 
+// A free node's update from the force on it: velocity, displacement, compensation, and the
+// step's external work and kinetic energy added to work / kin.
+template <bool KAHAN>
+__device__ __forceinline__ void tet_node_update(float m, float im, const float (&force)[3], const float (&ext)[3], float dt,
+                                                float damping, float* vel, float4& u4, float4& c4, double& work, double& kin) {
+    float* u = &u4.x;
+    float* cu = &c4.x;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        float v = vel[k] + (force[k] + ext[k]) * im * dt;
+        v *= damping;
+        vel[k] = v;
+        const float du = v * dt;
+        if (KAHAN)
+            kahan_add(u[k], cu[k], du);
+        else
+            u[k] += du;
+        work += (double)ext[k] * (double)v * (double)dt;
+        kin += 0.5 * (double)m * (double)v * (double)v;
+    }
+}
+
 // One node: `gather` adds the forces of its slots in order to its weight (it is not called
 // for a fixed node); external load, symplectic Euler on the displacement.
 template <bool KAHAN, class Gather>
@@ -438,21 +446,7 @@ __device__ __forceinline__ void tet_node_f32(const TetNodeRefs& d, Gather gather
     }
     const float im = d.inv_mass[n];
     float4 u4 = d.disp[n], c4 = KAHAN ? d.disp_c[n] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float* u = &u4.x;
-    float* cu = &c4.x;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        float v = vel[k] + (force[k] + ext[k]) * im * dt;
-        v *= damping;
-        vel[k] = v;
-        const float du = v * dt;
-        if (KAHAN)
-            kahan_add(u[k], cu[k], du);
-        else
-            u[k] += du;
-        work += (double)ext[k] * (double)v * (double)dt;
-        kin += 0.5 * (double)m * (double)v * (double)v;
-    }
+    tet_node_update<KAHAN>(m, im, force, ext, dt, damping, vel, u4, c4, work, kin);
     d.disp[n] = u4;
     if (KAHAN) d.disp_c[n] = c4;
     gwork = -(double)gravity * (double)m * (double)vel[2] * (double)dt;

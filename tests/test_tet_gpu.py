@@ -237,3 +237,47 @@ def test_uneven_runs_of_slots(fem, port, spokes):
     r.run(60, youngs=210e9, poisson=0.3, dt=dt, gravity=9.80665, damping=1.0)
     pr, vr = r.readback()
     assert np.array_equal(pr, m.position) and np.array_equal(vr, m.velocity)
+
+
+@pytest.mark.parametrize("mode", ["ref32", "f32", "f32k", "f64"])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (7, 3, 1), (43, 1, 1), (13, 9, 5), (11, 10, 6), (682, 1, 1), (21, 13, 5)])
+def test_cluster_run_is_the_steps_to_the_bit(fem, mode, cells):
+    """A long run of a small mesh is one launch of one cluster of blocks: 6 to 8,190 tets,
+    one to sixteen blocks of 128 to 512 threads, ragged last groups (FP64 above 4,096 tets
+    takes the two kernels a step).  State and energy account to the bit those of the same
+    steps in short runs, before and after it too."""
+    nx, ny, nz = cells
+    pos, idx = fem.box_tet_mesh(0.05 * nx, 0.05 * ny, 0.05 * nz, nx, ny, nz)
+    fixed = (pos[0::3] < 1e-6).astype(np.uint32)
+    tip = pos[0::3] > 0.05 * nx - 1e-6
+    fext = np.zeros(pos.size)
+    fext[2::3][tip] = -3e5 * ny * nz / max(1, tip.sum())  # the longest mesh's tip rounds away: gravity alone
+    if mode == "ref32":
+        x = pos.reshape(-1, 3).astype(np.float64)[idx.reshape(-1, 4)]
+        d = np.transpose(x[:, 1:] - x[:, :1], (0, 2, 1))
+        vol = np.abs(np.linalg.det(d)) / 6
+        off, ent = fem.csr(pos.size // 3, idx, 4)
+        mass = np.bincount(idx, weights=np.repeat(7850 * vol / 4, 4), minlength=pos.size // 3)
+        vel = np.zeros(pos.size)
+        vel[2::3] = -10.0 * pos[0::3]
+        kw = dict(mass=mass, velocity=vel, rest_volume=vol, adjacency_offset=off, adjacency_entry=ent,
+                  rest_inv=np.transpose(np.linalg.inv(d), (0, 2, 1)))
+    else:
+        kw = dict(external_force=fext, density=7850.0)
+    a, b = (fem.TetSolver(pos, idx, mode=mode, fixed=fixed, **kw) for _ in range(2))
+    run = dict(dt=1.5e-6, gravity=9.80665, damping=0.9999, ramp_steps=100)
+    a.run(7, **run)
+    a.run(200, **run)
+    used = a.launches
+    a.run(40, **run)
+    for n in (7, 50, 50, 50, 50, 40):
+        b.run(n, **run)
+    fits = idx.size // 4 <= (4096 if mode == "f64" else 8192)
+    assert used == (1 if fits else 400)
+    pa, va = a.readback64()
+    pb, vb = b.readback64()
+    assert np.abs(pa - pos).max() > 1e-7 and np.isfinite(pa).all()
+    assert np.array_equal(pa, pb) and np.array_equal(va, vb)
+    assert np.array_equal(a.plastic(), b.plastic()) and np.array_equal(a.energy(), b.energy())
+    if mode != "ref32" and nx > 10 and tip.any():
+        assert (a.plastic()[:, 6] > 0).any(), "the case must yield"
