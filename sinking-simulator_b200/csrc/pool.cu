@@ -42,7 +42,7 @@ __device__ __forceinline__ void element_tile(const PoolDevice& d, int tile, int 
     if (live && t < tl.end) tet_element_f32<true, CG>(element_refs(d), t, m.mat, diss, energy);
     block_sum2(diss, energy, scratch);  // valid in thread 0
     if (live && threadIdx.x == 0) {
-        if (diss != 0.0) d.e_diss[tl.part] += diss;  // else the sum stands, unread
+        account_add(&d.e_diss[tl.part], diss);
         d.e_strain[tl.part] = energy;
     }
 }
@@ -137,7 +137,7 @@ __device__ __forceinline__ void node_tile(const PoolDevice& d, int tile, int sub
     work += gwork;
     block_sum2(work, kin, scratch);  // valid in thread 0
     if (live && threadIdx.x == 0) {
-        d.n_work[tl.part] += work;
+        account_add(&d.n_work[tl.part], work);
         d.n_kin[tl.part] = kin;
     }
 }
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(B, MINB) pool_elements_ring(PoolDevice d, int 
         }
         block_sum2(diss, energy, scratch);  // valid in thread 0; also the closing barrier
         if (threadIdx.x == 0 && live && ok) {
-            if (diss != 0.0) d.e_diss[tl.part] += diss;  // else the sum stands, unread
+            account_add(&d.e_diss[tl.part], diss);
             d.e_strain[tl.part] = energy;
         }
         if (next >= d.n_etiles) break;

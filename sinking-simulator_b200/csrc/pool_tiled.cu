@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kTiledTile, 1024 / kTiledTile) pool_elements_t
                 diss += warp_sums[which][0][w];
                 energy += warp_sums[which][1][w];
             }
-            if (diss != 0.0) d.e_diss[info[which].part] += diss;  // else the sum stands, unread
+            account_add(&d.e_diss[info[which].part], diss);
             d.e_strain[info[which].part] = energy;
         }
     };

@@ -1198,10 +1198,9 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) energy += __shfl_xor_sync(0xffffffffu, energy, off);
     if (lane == 0) {
-        // sums that gain nothing stand as they are, unread
-        if (diss != 0.0) d.e_diss[group_raw] += diss;
+        account_add(&d.e_diss[group_raw], diss);
         d.e_strain[group_raw] = energy;
-        if (nonconv) d.e_stats[group_raw * 2] += __popc(nonconv);
+        if (nonconv) atomicAdd(&d.e_stats[group_raw * 2], __popc(nonconv));
         d.e_stats[group_raw * 2 + 1] = __popc(ypts);
     }
 }
@@ -1222,7 +1221,7 @@ __device__ __forceinline__ void shell_move(float* u, float* uc, float v, float d
 
 template <bool KAHAN>
 __global__ void __launch_bounds__(kShellNodeBlock) shell_nodes(ShellDevice d, ShellParams p) {
-    __shared__ double scratch[32];
+    __shared__ double scratch[64];
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long nr = n < d.nodes ? n : d.nodes - 1;
     const uint32_t b = d.offset[nr], e = d.offset[nr + 1];
@@ -1328,17 +1327,16 @@ __global__ void __launch_bounds__(kShellNodeBlock) shell_nodes(ShellDevice d, Sh
             }
         }
     }
-    const double bw = block_sum(work, scratch);
-    const double bk = block_sum(kin, scratch);
+    block_sum2(work, kin, scratch);  // valid in thread 0
     const double bp = d.driven && !p.inertial ? block_sum(pwork, scratch) : 0.0;
     const double bd = p.damping64 != 1.0 ? block_sum(damp, scratch) : 0.0;
     const double be = d.edge_map ? block_sum(bwork, scratch) : 0.0;
     if (threadIdx.x == 0) {
-        d.n_work[blockIdx.x] += bw;
-        d.n_kin[blockIdx.x] = bk;
-        if (d.driven && !p.inertial) d.n_punch[blockIdx.x] += bp;
-        if (p.damping64 != 1.0) d.n_damp[blockIdx.x] += bd;
-        if (d.edge_map) d.n_edge[blockIdx.x] += be;
+        account_add(&d.n_work[blockIdx.x], work);
+        d.n_kin[blockIdx.x] = kin;
+        if (d.driven && !p.inertial) account_add(&d.n_punch[blockIdx.x], bp);
+        if (p.damping64 != 1.0) account_add(&d.n_damp[blockIdx.x], bd);
+        if (d.edge_map) account_add(&d.n_edge[blockIdx.x], be);
     }
 }
 
@@ -1459,7 +1457,7 @@ __global__ void __launch_bounds__(kShellFiberBlock) shell_fibers(ShellDevice d, 
     }
     block_sum2(diss, energy, scratch);
     if (threadIdx.x == 0) {
-        d.f_diss[blockIdx.x] += diss;
+        account_add(&d.f_diss[blockIdx.x], diss);
         d.f_energy[blockIdx.x] = energy;
     }
 }

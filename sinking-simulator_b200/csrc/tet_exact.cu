@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(kTet64Block, 5) f64_forces(TetDevice<double> d
     f64_element<false>(d, p, park, t, live, idx, diss, energy);
     block_sum2(diss, energy, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
-        if (diss != 0.0) d.e_diss[blockIdx.x] += diss;  // else the sum stands, unread
+        account_add(&d.e_diss[blockIdx.x], diss);
         d.e_strain[blockIdx.x] = energy;
     }
 }
@@ -638,12 +638,12 @@ __global__ void __launch_bounds__(kTetNodeBlock) f64_nodes(TetDevice<double> d, 
     }
     block_sum2(work, kin, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
-        d.n_work[blockIdx.x] += work;
+        account_add(&d.n_work[blockIdx.x], work);
         d.n_kin[blockIdx.x] = kin;
     }
     if (p.gravity != 0.0) {
         gwork = block_sum(gwork, scratch);
-        if (threadIdx.x == 0) d.n_grav[blockIdx.x] += gwork;
+        if (threadIdx.x == 0) account_add(&d.n_grav[blockIdx.x], gwork);
     }
 }
 

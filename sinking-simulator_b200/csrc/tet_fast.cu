@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(kTetF32Block, 1024 / kTetF32Block) f32_forces(
     if (t < d.tets) tet_element_f32<KAHAN, false, LoadedRows>(r, rows, t, m, diss, energy);
     block_sum2(diss, energy, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
-        if (diss != 0.0) d.e_diss[blockIdx.x] += diss;  // else the sum stands, unread
+        account_add(&d.e_diss[blockIdx.x], diss);
         d.e_strain[blockIdx.x] = energy;
     }
 }
@@ -83,12 +83,12 @@ __global__ void __launch_bounds__(kTetNodeBlock) f32_nodes(TetDevice<float> d, f
     }
     block_sum2(work, kin, scratch);  // valid in thread 0
     if (threadIdx.x == 0) {
-        d.n_work[blockIdx.x] += work;
+        account_add(&d.n_work[blockIdx.x], work);
         d.n_kin[blockIdx.x] = kin;
     }
     if (gravity != 0.0f) {
         gwork = block_sum(gwork, scratch);
-        if (threadIdx.x == 0) d.n_grav[blockIdx.x] += gwork;
+        if (threadIdx.x == 0) account_add(&d.n_grav[blockIdx.x], gwork);
     }
 }
 
