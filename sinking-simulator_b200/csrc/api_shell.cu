@@ -331,6 +331,13 @@ int femstep_shell_create(const femstep_shell_mesh* mesh, femstep_shell** out) {
     d.e_diss = A.zeros<double>(s->ewarps);
     d.e_strain = A.zeros<double>(s->ewarps);
     d.e_stats = A.zeros<int>((size_t)s->ewarps * 2);
+    if (fs::shell_wide(s->groups, d.sms) && s->groups <= fs::kShellOrderMost) {
+        std::vector<uint16_t> order((size_t)s->ewarps);
+        for (size_t k = 0; k < order.size(); ++k) order[k] = (uint16_t)k;
+        d.order = A.upload(order.data(), order.size());
+        d.cost = A.zeros<uint8_t>((size_t)s->ewarps);
+        d.ordered = A.zeros<int>(1);
+    }
     s->kaa_factor = A.zeros<float>(E * 32);
     d.n_work = A.zeros<double>(s->nblocks);
     d.n_kin = A.zeros<double>(s->nblocks + 1);  // + the gripped nodes of an inertial punch
@@ -548,7 +555,7 @@ int femstep_shell_run(femstep_shell* s, int substeps, const femstep_shell_params
             cudaGraph_t g = nullptr;
             rc = check(s, cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "capture");
             if (rc) return rc;
-            for (int i = 0; i < kGraphSteps; ++i) fs::launch_shell_step(s->d, q, s->stream, 3);
+            for (int i = 0; i < kGraphSteps; ++i) fs::launch_shell_step(s->d, q, s->stream, 3, i + 1 == kGraphSteps);
             rc = check(s, cudaStreamEndCapture(s->stream, &g), "capture end");
             if (rc) return rc;
             rc = check(s, cudaGraphInstantiate(&s->graph, g, 0), "graph instantiate");

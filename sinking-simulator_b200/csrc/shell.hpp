@@ -102,6 +102,11 @@ struct ShellDevice {
     double* n_work = nullptr;         // += per node block
     double* n_kin = nullptr;          // =
     int* e_stats = nullptr;           // per element warp: [0] += non-converged, [1] = yielded points
+    // a zone of a few waves: the groups in the order the warps take them, and each one's
+    // Newton iterations in the last step (shell_order); else null
+    uint16_t* order = nullptr;        // [element warps]
+    uint8_t* cost = nullptr;          // [element warps]
+    int* ordered = nullptr;           // 0: the order is the mesh's
 };
 
 struct ShellParams {
@@ -154,7 +159,12 @@ constexpr int kShellNodeBlock = 256;
 constexpr int kShellPunchBlock = 256;   // the inertial punch: one block
 constexpr int kShellFiberBlock = 128;
 
-void launch_shell_step(const ShellDevice& d, const ShellParams& p, cudaStream_t stream, int parts);
+// `sort`: the node pass also brings ShellDevice::order up to date (where there is one).
+void launch_shell_step(const ShellDevice& d, const ShellParams& p, cudaStream_t stream, int parts, bool sort = false);
+// The largest zone (in groups of four elements) whose warps are ordered, and whether the
+// wide form of the element pass takes a zone.
+constexpr long long kShellOrderMost = 16384;
+bool shell_wide(long long groups, int sms);
 // Factor of the elastic K_aa per element for this material (into `out`, [E][32]).
 void launch_shell_elastic_factor(const ShellDevice& d, double youngs, double poisson, float* out,
                                  cudaStream_t stream);

@@ -562,3 +562,29 @@ def test_zone_inputs_are_checked(fem):
     s.run(16, dt=float(g["dt"]))
     p, v = s.readback()
     assert np.array_equal(p, g["rest"]) and not np.abs(v).any()
+
+
+@pytest.mark.parametrize("law", ["linear", "swift"])
+@pytest.mark.parametrize("nx,ny", [(37, 193), (90, 80), (259, 253)])
+def test_ordered_warps_change_no_bits(fem, nx, ny, law):
+    """A zone of a few waves takes its groups of elements in an order renewed once a graph of
+    16 steps: 7,141 elements (one over a group), 7,200 and 65,527 (the largest ordered zone
+    less a corner of its last group).  State and account to the bit those of single steps,
+    which keep the mesh's order."""
+    rest, index, pinned, load = fem.stiffened_panel(nx=nx, ny=ny, lx=0.01 * nx, ly=0.01 * ny, thickness=0.008,
+                                                    stiffeners=0, imperfection=2e-4, peak_pressure=4e7, radius=10.0)
+    params = dict(rise_time=2e-5, max_iterations=12, damping=0.9999)
+    if law == "swift":
+        params["material"] = dict(hardening=fem.SHELL_SWIFT, strength_coefficient=600e6, reference_strain=0.02,
+                                  hardening_exponent=0.18)
+    a, b = (fem.ShellSolver(rest, index, pinned=pinned, load=load, density=7850.0) for _ in range(2))
+    dt = a.critical_dt(206e9, 0.3, 7850.0, 0.8)
+    for n in (48, 5, 32):
+        a.run(n, dt=dt, **params)
+        for _ in range(n):
+            b.run(1, dt=dt, **params)
+    assert (a.state()[:, 12:120:15] > 0).sum() > 100, "the case must yield"
+    assert np.array_equal(a.state(), b.state()) and np.array_equal(a.energy(), b.energy())
+    for x, y in zip(a.readback(), b.readback()):
+        assert np.array_equal(x, y)
+    assert a.stats() == b.stats()
