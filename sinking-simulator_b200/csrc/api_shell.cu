@@ -94,6 +94,7 @@ ShellParams make_params(const femstep_shell_params& p) {
     q.kappa = (float)kappa;
     q.yield = (float)p.yield_strength;
     q.hardening = (float)p.hardening_modulus;
+    q.theta_bar = 1.0f / (1.0f + q.hardening / (3.0f * q.mu));
     q.dt = (float)p.dt;
     q.dt64 = p.dt;
     q.damping = (float)p.damping;

@@ -111,6 +111,7 @@ struct ShellDevice {
 
 struct ShellParams {
     float mu, kappa, yield, hardening;   // J2 point law, linear isotropic hardening
+    float theta_bar;                      // 1 / (1 + hardening / (3 mu)): the tangent's, linear curve
     // The general point law of plasticity::update (plasticity.cpp:319-505): a Swift
     // curve K (eps0 + p)^n instead of the linear one, linear kinematic hardening (back
     // stress), ductile damage D += d(eps_p) / (eps_f f(eta)) with eps_f the element's
