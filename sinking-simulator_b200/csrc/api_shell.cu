@@ -10,7 +10,9 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/femstep.h"
@@ -29,6 +31,7 @@ struct femstep_shell {
     fs::DeviceArena arena;
     ShellDevice d;
     int eblocks = 0, nblocks = 0;
+    float* pinned_slices = nullptr;   // kReadWorkers x 2 x kReadSlice: the readback's, made at its first use
     long long ewarps = 0;             // element-kernel warps = per-warp partial entries
     float* kaa_factor = nullptr;      // [E][32] elastic K_aa factor, for factor_E / factor_nu
     double factor_E = 0.0, factor_nu = 0.0;
@@ -141,6 +144,57 @@ ShellParams make_params(const femstep_shell_params& p) {
 }
 
 constexpr int kGraphSteps = 16;
+
+// The readback of a large zone, in slices: each worker copies a slice into its own pinned
+// buffer and widens it into the caller's array, whose pages it is often the first to touch,
+// while the others' copies run.  Two serial pageable copies and a widening pass each took 65
+// ms for the 4 M nodes of the panel, this 23 ms; under kReadParallel values there are too
+// few slices for the workers to share.
+constexpr size_t kReadWorkers = 16, kReadSlice = size_t(1) << 17, kReadParallel = size_t(1) << 21;
+
+int read_slices(femstep_shell* s, double* position, double* velocity) {
+    const size_t n3 = s->nodes * 3;
+    int device = 0;
+    cudaGetDevice(&device);
+    // the workers' streams wait for nobody's
+    int rc = check(s, cudaStreamSynchronize(cudaStreamLegacy), "readback");
+    if (!rc) rc = check(s, cudaStreamSynchronize(s->stream), "readback");
+    if (rc) return rc;
+    std::atomic<size_t> next{0};
+    std::atomic<int> failed{cudaSuccess};
+    const size_t each = (n3 + kReadSlice - 1) / kReadSlice, first = position ? 0 : each, last = velocity ? 2 * each : each;
+    next = first;
+    const auto work = [&](size_t w) {
+        float* a = s->pinned_slices + w * 2 * kReadSlice;
+        float* c = a + kReadSlice;
+        cudaStream_t stream = nullptr;
+        cudaError_t e = cudaSetDevice(device);
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        for (size_t k; e == cudaSuccess && failed == cudaSuccess && (k = next++) < last;) {
+            const size_t b = k % each * kReadSlice, n = std::min(kReadSlice, n3 - b), bytes = n * sizeof(float);
+            const bool moved = k < each;  // a slice of the positions, else of the velocities
+            e = cudaMemcpyAsync(a, (moved ? s->d.disp : s->d.velocity) + b, bytes, cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess && moved) e = cudaMemcpyAsync(c, s->d.disp_c + b, bytes, cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+            if (e != cudaSuccess) break;
+            if (moved)  // the compensated displacement u - c (c stays 0 without compensation)
+                for (size_t i = 0; i < n; ++i) position[b + i] = s->rest[b + i] + ((double)a[i] - (double)c[i]);
+            else
+                for (size_t i = 0; i < n; ++i) velocity[b + i] = a[i];
+        }
+        if (stream) cudaStreamDestroy(stream);
+        if (e != cudaSuccess) failed = e;
+    };
+    const size_t workers = std::min<size_t>(kReadWorkers, std::max(1u, std::thread::hardware_concurrency()));
+    std::vector<std::thread> pool;
+    try {  // with as many as can be had: this thread alone reads everything too
+        for (size_t w = 1; w < workers; ++w) pool.emplace_back(work, w);
+    } catch (const std::exception&) {
+    }
+    work(0);
+    for (auto& t : pool) t.join();
+    return check(s, (cudaError_t)failed.load(), "readback");
+}
 
 // The elastic K_aa factor depends on the material: formed before the first run and
 // again whenever E or nu change.
@@ -588,6 +642,11 @@ int femstep_shell_run(femstep_shell* s, int substeps, const femstep_shell_params
 int femstep_shell_readback(femstep_shell* s, double* position, double* velocity) {
     if (!s) return fail(s, FEMSTEP_EINVAL, "null solver");
     const size_t n3 = s->nodes * 3;
+    if (n3 >= kReadParallel && (position || velocity) &&
+        (s->pinned_slices || cudaHostAlloc((void**)&s->pinned_slices, kReadWorkers * 2 * kReadSlice * sizeof(float),
+                                           cudaHostAllocPortable) == cudaSuccess))
+        return read_slices(s, position, velocity);
+    cudaGetLastError();
     std::vector<float> buf(n3);
     int rc = FEMSTEP_OK;
     if (position) {
@@ -1177,6 +1236,7 @@ void femstep_shell_destroy(femstep_shell* s) {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->graph) cudaGraphExecDestroy(s->graph);
+    if (s->pinned_slices) cudaFreeHost(s->pinned_slices);
     s->arena.release();
     if (s->ev0) cudaEventDestroy(s->ev0);
     if (s->ev1) cudaEventDestroy(s->ev1);

@@ -514,6 +514,42 @@ int displacement(femstep_tet* s, std::vector<double>& out) {
     return FEMSTEP_OK;
 }
 
+// The FP32 modes' positions, rest + (u - c) in double, as Out.
+template <class Out>
+__global__ void f32_positions(const float4* disp, const float4* disp_c, const float* rest, long long nodes, Out* out) {
+    const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= nodes) return;
+    const float4 u = disp[n], c = disp_c ? disp_c[n] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    out[n * 3] = (Out)((double)rest[n * 3] + ((double)u.x - (double)c.x));
+    out[n * 3 + 1] = (Out)((double)rest[n * 3 + 1] + ((double)u.y - (double)c.y));
+    out[n * 3 + 2] = (Out)((double)rest[n * 3 + 2] + ((double)u.z - (double)c.z));
+}
+
+// They go to the caller formed on the device, in one copy without padding; where the device
+// has no room for them, they are formed here from the two padded arrays (88,641 nodes:
+// positions and velocities in 1.9 ms so, 1.0 ms from the device).
+template <class Out>
+int read_positions(femstep_tet* s, Out* position) {
+    const size_t n3 = s->nodes * 3;
+    void* out = nullptr;
+    if (fs::device_alloc(&out, n3 * sizeof(Out)) == cudaSuccess) {  // (which waits for the legacy stream)
+        f32_positions<Out><<<fs::blocks_for((long long)s->nodes, 256), 256, 0, s->stream>>>(
+            reinterpret_cast<const float4*>(s->d32.disp), reinterpret_cast<const float4*>(s->d32.disp_c), s->d32.rest,
+            (long long)s->nodes, static_cast<Out*>(out));
+        int rc = check(s, cudaGetLastError(), "readback");
+        if (!rc)
+            rc = check(s, cudaMemcpyAsync(position, out, n3 * sizeof(Out), cudaMemcpyDeviceToHost, s->stream), "readback");
+        if (!rc) rc = check(s, cudaStreamSynchronize(s->stream), "readback");
+        fs::device_free(out);
+        return rc;
+    }
+    cudaGetLastError();
+    std::vector<double> u;
+    const int rc = displacement(s, u);
+    for (size_t i = 0; i < n3 && !rc; ++i) position[i] = (Out)((double)s->rest[i] + u[i]);
+    return rc;
+}
+
 }  // namespace
 
 extern "C" {
@@ -537,9 +573,7 @@ int femstep_tet_readback(femstep_tet* s, float* position, float* velocity) {
         if (s->mode == FEMSTEP_TET_REF32) {
             rc = check(s, cudaMemcpy(position, s->d32.position, n3 * sizeof(float), cudaMemcpyDeviceToHost), "readback");
         } else {
-            std::vector<double> u;
-            rc = displacement(s, u);
-            for (size_t i = 0; i < n3 && !rc; ++i) position[i] = (float)((double)s->rest[i] + u[i]);
+            rc = read_positions(s, position);
         }
         if (rc) return rc;
     }
@@ -565,9 +599,7 @@ int femstep_tet_readback_f64(femstep_tet* s, double* position, double* velocity)
             rc = check(s, cudaMemcpy(p.data(), s->d32.position, n3 * sizeof(float), cudaMemcpyDeviceToHost), "readback");
             for (size_t i = 0; i < n3 && !rc; ++i) position[i] = p[i];
         } else {
-            std::vector<double> u;
-            rc = displacement(s, u);
-            for (size_t i = 0; i < n3 && !rc; ++i) position[i] = (double)s->rest[i] + u[i];
+            rc = read_positions(s, position);
         }
         if (rc) return rc;
     }

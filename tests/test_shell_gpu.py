@@ -588,3 +588,20 @@ def test_ordered_warps_change_no_bits(fem, nx, ny, law):
     for x, y in zip(a.readback(), b.readback()):
         assert np.array_equal(x, y)
     assert a.stats() == b.stats()
+
+
+@pytest.mark.parametrize("nx,ny", [(9, 7), (700, 497), (701, 499)])
+def test_readback_in_slices(fem, nx, ny):
+    """A large zone (from 2^21 values: 698,196 nodes just under it, 702,000 over, with a
+    ragged last slice) is read back in slices by several threads: the position and velocity
+    handed in come back, alone and together."""
+    rest, index, pinned, load = fem.stiffened_panel(nx=nx, ny=ny, lx=0.01 * nx, ly=0.01 * ny, thickness=0.008,
+                                                    stiffeners=0, imperfection=2e-4, peak_pressure=4e5, radius=1.0)
+    rng = np.random.default_rng(3)
+    pos = rest + rng.normal(0.0, 1e-3, rest.size)
+    vel = rng.normal(0.0, 1.0, rest.size).astype(np.float32).astype(np.float64)
+    s = fem.ShellSolver(rest, index, pinned=pinned, load=load, density=7850.0, position=pos, velocity=vel)
+    p, v = s.readback()
+    assert np.abs(p - pos).max() <= 1e-3 * 2.0 ** -40 and np.array_equal(v, vel)
+    q, w = s.readback()
+    assert np.array_equal(p, q) and np.array_equal(v, w)
