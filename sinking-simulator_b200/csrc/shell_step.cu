@@ -535,7 +535,9 @@ __device__ __forceinline__ bool shell_row(const float4* row, float (&j0)[9], flo
 // 2.34 ms, 6 (85 registers, ~650 bytes) 2.74 ms.  A zone that fits in one wave is
 // bound by one warp's dependent chain, where every spill reload is latency: on the
 // reference's 2,048-element probe zone 3 blocks (168 registers, no spill) take 18.2 us
-// per step, 4 blocks 19.7 us, 5 blocks 24.0 us.
+// per step, 4 blocks 19.7 us, 5 blocks 24.0 us.  (All measured before the wide form's
+// state, frames and factor waited in shared memory: at 5 blocks, 130 bytes of spill, the
+// panel's pass takes 1.27 ms now.)
 constexpr int kShellMinbWide = 5;
 constexpr int kShellMinbNarrow = 3;
 constexpr int kShellWarpsNarrow = kShellMinbNarrow * kShellBlock / 32;  // per SM
