@@ -255,6 +255,7 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         s->inv64 = inv64;
     }
     if (!rc) rc = check(s, cudaStreamSynchronize(s->stream), "set-up");
+    if (!rc) rc = check(s, cudaStreamSynchronize(cudaStreamLegacy), "upload");  // the last uploads, before any step
     fs::device_free(entry);
     fs::device_free(offset);
     fs::device_free(quarter);
@@ -350,6 +351,9 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
         if (!rc) rc = check(s, fs::device_alloc((void**)&dentry, T * 4 * sizeof(uint32_t)), "alloc");
         if (!rc) rc = check(s, cudaMemcpy(doffset, offset.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
         if (!rc) rc = check(s, cudaMemcpy(dentry, entry.data(), T * 4 * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
+        // (a copy from pageable memory may return before it has landed, and the solver's
+        // stream does not wait for the legacy one)
+        if (!rc) rc = check(s, cudaStreamSynchronize(cudaStreamLegacy), "upload");
         if (!rc && A.ok())
             rc = check(s, fs::build_runs_device(doffset, dentry, (long long)T * 4, (long long)N, run, slot, &slots, s->stream),
                        "slot runs");
@@ -439,6 +443,11 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
         fail(s, code, std::string("device upload failed: ") + cudaGetErrorString(A.status()));
         femstep_tet_destroy(s);
         return code;
+    }
+    rc = check(s, cudaStreamSynchronize(cudaStreamLegacy), "upload");  // the last uploads, before any step
+    if (rc) {
+        femstep_tet_destroy(s);
+        return rc;
     }
     *out = s;
     return FEMSTEP_OK;

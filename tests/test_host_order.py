@@ -1,0 +1,71 @@
+"""What the host code orders before what, without a GPU: the library's own objects linked
+with fake_cudart.cpp, where no kernel runs and device work stays pending until something
+waits for it."""
+import ctypes as C
+import glob
+import importlib.util
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "sinking-simulator_b200")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def bound(tmp_path_factory):
+    """The binding over the library's host code and the fake runtime."""
+    subprocess.run(["make", "-s", "-C", PKG, "-j8"], check=True)
+    so = str(tmp_path_factory.mktemp("fake") / "libfemstep_fake.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-Wl,--no-undefined",
+                    "-I", os.path.join(CUDA, "include"), os.path.join(ROOT, "tests", "fake_cudart.cpp"),
+                    *sorted(glob.glob(os.path.join(PKG, "_build", "*.o"))), "-o", so, "-lpthread"], check=True)
+    spec = importlib.util.spec_from_file_location("femstep_fake", os.path.join(PKG, "femstep.py"))
+    module = importlib.util.module_from_spec(spec)
+    real = C.CDLL
+    C.CDLL = lambda path, *a, **k: real(so, *a, **k)
+    try:
+        spec.loader.exec_module(module)
+    finally:
+        C.CDLL = real
+    return module
+
+
+@pytest.fixture
+def fake(bound):
+    bound.lib.fake_reset()
+    return bound
+
+
+def tet_case(fem, mode, adjacency, cells=(4, 2, 2), load=True):
+    pos, idx = fem.box_tet_mesh(0.4, 0.1, 0.02, *cells)
+    N, T = pos.size // 3, idx.size // 4
+    kw = {}
+    if mode == "ref32":
+        kw = dict(mass=np.ones(N), rest_inv=np.ones((T, 9)), rest_volume=np.ones(T))
+    else:
+        kw = dict(density=7850.0)
+        if load:
+            kw["external_force"] = np.ones(N * 3)
+    if adjacency:
+        kw["adjacency_offset"], kw["adjacency_entry"] = fem.csr(N, idx, 4)
+    return pos, idx, dict(kw, mode=mode, fixed=np.zeros(N, np.uint32), velocity=np.zeros(N * 3))
+
+
+@pytest.mark.parametrize("load", [True, False])
+@pytest.mark.parametrize("adjacency", [True, False])
+@pytest.mark.parametrize("mode", ["ref32", "f32", "f32k", "f64"])
+def test_tet_uploads_land_before_the_solver_reads_them(fake, mode, adjacency, load):
+    """A copy from pageable memory and a memset on the legacy stream may return before the
+    device has done them, and the solver's stream does not wait for that stream: both are
+    waited for before a set-up kernel and before create returns."""
+    pos, idx, kw = tet_case(fake, mode, adjacency, load=load)
+    s = fake.TetSolver(pos, idx, **kw)
+    assert fake.lib.fake_unordered() == 0
+    assert fake.lib.fake_pending() == 0
+    s.run(40, dt=1e-6)
+    assert fake.lib.fake_unordered() == 0
+    s.close()
