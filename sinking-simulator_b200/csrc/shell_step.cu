@@ -727,17 +727,18 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
 #pragma unroll
         for (int i = 0; i < 3; ++i)
             geo[kGeoU + gp * 3 + i] = ddg[i] + (q[0 * 3 + i] * sx + q[1 * 3 + i] * ty + q[2 * 3 + i] * wz);
+        // the rotation waits in shared memory through the Newton iterations, freeing nine
+        // registers there; stored here, ahead of the synchronisation, because the other lanes
+        // read it and a warp that is done at its first test passes no other
+        if constexpr (!PARK) {
+            if (gp == 0) {
+#pragma unroll
+                for (int k = 0; k < 9; ++k) geo[kGeoQ + k] = q[k];
+            }
+        }
         __syncwarp();
     }
 
-    // the rotation waits in shared memory through the Newton iterations, freeing nine
-    // registers there
-    if constexpr (!PARK) {
-        if (gp == 0) {
-#pragma unroll
-            for (int k = 0; k < 9; ++k) geo[kGeoQ + k] = q[k];
-        }
-    }
     // ---- the point's operators, formed from the rest geometry ----
     const ShellLanePoint P = shell_lane_point(gp);
     float w, eps_u[6];
