@@ -625,8 +625,8 @@ int femstep_shell_run(femstep_shell* s, int substeps, const femstep_shell_params
             s->launches += per_step * kGraphSteps;
         }
     }
-    for (; left > 0; --left) {
-        fs::launch_shell_step(s->d, q, s->stream, 3);
+    for (bool early = left == substeps; left > 0; --left, early = true) {  // the first waits for a graph before it
+        fs::launch_shell_step(s->d, q, s->stream, 3, false, early);
         s->launches += per_step;
     }
     rc = check(s, cudaGetLastError(), "kernel launch");

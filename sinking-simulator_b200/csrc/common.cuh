@@ -30,8 +30,12 @@ inline int sm_count() {
 // evenly (among the node pass's blocks the 256-mesh batch's step took 772 us for 563), and
 // node blocks that come up beside an element pass run with its shared-memory carve-out
 // and little L1 (the staged schedule on 12 meshes: 98 us for 58).
+//
+// launch_kernel: `early`, or else as an ordinary launch, which starts once all before it in the
+// stream is complete.
 template <class... Params, class... Args>
-inline void launch_pdl(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, Args... args) {
+inline void launch_kernel(bool early, void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream,
+                        Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
@@ -41,8 +45,12 @@ inline void launch_pdl(void (*kernel)(Params...), int grid, int block, size_t sm
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+template <class... Params, class... Args>
+inline void launch_pdl(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t stream, Args... args) {
+    launch_kernel(true, kernel, grid, block, smem, stream, args...);
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

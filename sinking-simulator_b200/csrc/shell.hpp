@@ -160,8 +160,11 @@ constexpr int kShellNodeBlock = 256;
 constexpr int kShellPunchBlock = 256;   // the inertial punch: one block
 constexpr int kShellFiberBlock = 128;
 
-// `sort`: the node pass also brings ShellDevice::order up to date (where there is one).
-void launch_shell_step(const ShellDevice& d, const ShellParams& p, cudaStream_t stream, int parts, bool sort = false);
+// `sort`: the node pass also brings ShellDevice::order up to date (where there is one).  The
+// element pass reads the order before it waits for the pass ahead of it, so the step after
+// one that sorts is not launched `early` (as a programmatic dependent).
+void launch_shell_step(const ShellDevice& d, const ShellParams& p, cudaStream_t stream, int parts, bool sort = false,
+                       bool early = true);
 // The largest zone (in groups of four elements) whose warps are ordered, and whether the
 // wide form of the element pass takes a zone.
 constexpr long long kShellOrderMost = 16384;

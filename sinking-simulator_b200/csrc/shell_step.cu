@@ -553,7 +553,8 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
     const int gp = lane & 7;
     long long group_raw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if constexpr (MINB >= kShellMinbWide) {
-        // (both are rewritten only before a launch that waits for it)
+        // (rewritten only by the last step of a graph of steps: the launch after a graph waits
+        // for all of it)
         if (d.order && *d.ordered) group_raw = d.order[group_raw];
     }
     const long long e_raw = group_raw * 4 + (lane >> 3);
@@ -1328,12 +1329,16 @@ __global__ void __launch_bounds__(kShellNodeBlock) shell_nodes(ShellDevice d, Sh
     const uint8_t pin = d.pinned[nr];
     const float im = d.inv_mass[nr], m = d.mass[nr];
     pdl_wait();
-    pdl_next();
-    if (d.halt && *d.halt) return;  // an inertial punch has stopped: the run is over
+    const bool halted = d.halt && *d.halt;  // an inertial punch has stopped: the run is over
     if (SORT && blockIdx.x == gridDim.x - 1) {
-        shell_order(d.cost, d.order, d.ordered, (int)(d.groups + kShellBlock / 32 - 1) / (kShellBlock / 32) * (kShellBlock / 32));
+        // no pdl_next(): the next kernel comes up once this block has ended, its order written
+        if (!halted)
+            shell_order(d.cost, d.order, d.ordered,
+                        (int)(d.groups + kShellBlock / 32 - 1) / (kShellBlock / 32) * (kShellBlock / 32));
         return;
     }
+    pdl_next();
+    if (halted) return;
     double work = 0.0, kin = 0.0, pwork = 0.0, damp = 0.0, bwork = 0.0;
     if (n < d.nodes) {
         const double t = (double)(d.counter[1] + 1) * p.dt64;  // the time at the step's end
@@ -1720,52 +1725,54 @@ void launch_shell_elastic_factor(const ShellDevice& d, double youngs, double poi
 }
 
 template <int MINB>
-static void launch_forces(const ShellDevice& d, const ShellParams& p, int blocks, cudaStream_t stream) {
+static void launch_forces(const ShellDevice& d, const ShellParams& p, int blocks, cudaStream_t stream, bool early) {
     // the FP64 enhanced-block variants: compensated state and the general law only (the
     // host checks), at the narrow register budget
     if (p.eas64 == 1) {
-        launch_pdl(shell_forces<true, true, kShellMinbNarrow, 1>, blocks, kShellBlock, 0, stream, d, p);
+        launch_kernel(early, shell_forces<true, true, kShellMinbNarrow, 1>, blocks, kShellBlock, 0, stream, d, p);
         return;
     }
     if (p.eas64 == 2) {
-        launch_pdl(shell_forces<true, true, kShellMinbNarrow, 2>, blocks, kShellBlock, 0, stream, d, p);
+        launch_kernel(early, shell_forces<true, true, kShellMinbNarrow, 2>, blocks, kShellBlock, 0, stream, d, p);
         return;
     }
     if (p.eas64 == 3) {
-        launch_pdl(shell_forces<true, true, kShellMinbNarrow, 3>, blocks, kShellBlock, 0, stream, d, p);
+        launch_kernel(early, shell_forces<true, true, kShellMinbNarrow, 3>, blocks, kShellBlock, 0, stream, d, p);
         return;
     }
     if (p.compensated) {
         if (p.general)
-            launch_pdl(shell_forces<true, true, MINB>, blocks, kShellBlock, 0, stream, d, p);
+            launch_kernel(early, shell_forces<true, true, MINB>, blocks, kShellBlock, 0, stream, d, p);
         else
-            launch_pdl(shell_forces<true, false, MINB>, blocks, kShellBlock, 0, stream, d, p);
+            launch_kernel(early, shell_forces<true, false, MINB>, blocks, kShellBlock, 0, stream, d, p);
     } else {
         if (p.general)
-            launch_pdl(shell_forces<false, true, MINB>, blocks, kShellBlock, 0, stream, d, p);
+            launch_kernel(early, shell_forces<false, true, MINB>, blocks, kShellBlock, 0, stream, d, p);
         else
-            launch_pdl(shell_forces<false, false, MINB>, blocks, kShellBlock, 0, stream, d, p);
+            launch_kernel(early, shell_forces<false, false, MINB>, blocks, kShellBlock, 0, stream, d, p);
     }
 }
 
 bool shell_wide(long long groups, int sms) { return groups > (long long)sms * kShellWarpsNarrow; }
 
-void launch_shell_step(const ShellDevice& d, const ShellParams& p, cudaStream_t stream, int parts, bool sort) {
+void launch_shell_step(const ShellDevice& d, const ShellParams& p, cudaStream_t stream, int parts, bool sort,
+                       bool early) {
     const int eb = blocks_for(d.groups * 32, kShellBlock);
     const int nb = blocks_for(d.nodes, kShellNodeBlock);
     const int fb = blocks_for(d.fibers, kShellFiberBlock);
     if ((parts & 1) && d.fibers) {
         if (p.compensated)
-            launch_pdl(shell_fibers<true>, fb, kShellFiberBlock, 0, stream, d, p);
+            launch_kernel(early, shell_fibers<true>, fb, kShellFiberBlock, 0, stream, d, p);
         else
-            launch_pdl(shell_fibers<false>, fb, kShellFiberBlock, 0, stream, d, p);
+            launch_kernel(early, shell_fibers<false>, fb, kShellFiberBlock, 0, stream, d, p);
+        early = true;  // the element pass follows that one
     }
     // one wave at the narrow budget: the latency-bound form; else the wide one
     if (parts & 1) {
         if (shell_wide(d.groups, d.sms))
-            launch_forces<kShellMinbWide>(d, p, eb, stream);
+            launch_forces<kShellMinbWide>(d, p, eb, stream, early);
         else
-            launch_forces<kShellMinbNarrow>(d, p, eb, stream);
+            launch_forces<kShellMinbNarrow>(d, p, eb, stream, early);
     }
     sort = sort && d.order;
     if (p.compensated) {

@@ -69,3 +69,22 @@ def test_tet_uploads_land_before_the_solver_reads_them(fake, mode, adjacency, lo
     s.run(40, dt=1e-6)
     assert fake.lib.fake_unordered() == 0
     s.close()
+
+
+def shell_zone(fem, nx, ny):
+    rest, index, pinned, load = fem.stiffened_panel(nx=nx, ny=ny, lx=0.01 * nx, ly=0.01 * ny, thickness=0.008,
+                                                    stiffeners=0, imperfection=2e-4, peak_pressure=4e7, radius=10.0)
+    return fem.ShellSolver(rest, index, pinned=pinned, load=load, density=7850.0)
+
+
+@pytest.mark.parametrize("fibres", [False, True])
+def test_shell_step_after_a_graph_waits_for_it(fake, fibres):
+    """The last step of a graph renews the order that an element pass reads as soon as it comes
+    up: a direct step right after a graph is an ordinary launch."""
+    s = shell_zone(fake, 90, 80)
+    if fibres:
+        s.set_fibers([[0, 8281, 1, 8282]], [[0.5, 0.5]], [1e-4])
+    for n in (37, 16, 5):
+        s.run(n, dt=1e-7)
+        assert fake.lib.fake_early_after_graph() == 0
+    s.close()

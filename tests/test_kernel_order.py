@@ -31,3 +31,11 @@ def test_shell_rotation_is_synchronised_before_its_readers():
     sync = after.index("__syncwarp();")
     assert sync < after.index("load_record<"), "the rotation is stored after the last synchronisation"
     assert sync < after.index("geo[kGeoQ + k]")
+
+
+def test_shell_order_is_written_before_the_next_kernel_may_start():
+    """The element pass reads the order of its groups before it waits for the pass ahead, so
+    the block that renews it must not let the next kernel start first."""
+    body = kernel("shell_step.cu", "shell_nodes")
+    assert "pdl_next();" in body
+    assert "pdl_next();" not in body[:body.index("shell_order(")]

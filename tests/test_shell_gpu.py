@@ -605,3 +605,23 @@ def test_readback_in_slices(fem, nx, ny):
     assert np.abs(p - pos).max() <= 1e-3 * 2.0 ** -40 and np.array_equal(v, vel)
     q, w = s.readback()
     assert np.array_equal(p, q) and np.array_equal(v, w)
+
+
+@pytest.mark.parametrize("nx,ny", [(37, 193), (90, 80)])
+def test_ordered_warps_from_a_graph_into_direct_steps(fem, nx, ny):
+    """The same in runs that go from graphs of 16 steps straight into direct ones, where the
+    order was renewed by the launch just before: to the bit those of single steps."""
+    rest, index, pinned, load = fem.stiffened_panel(nx=nx, ny=ny, lx=0.01 * nx, ly=0.01 * ny, thickness=0.008,
+                                                    stiffeners=0, imperfection=2e-4, peak_pressure=4e7, radius=10.0)
+    params = dict(rise_time=2e-5, max_iterations=12, damping=0.9999)
+    a, b = (fem.ShellSolver(rest, index, pinned=pinned, load=load, density=7850.0) for _ in range(2))
+    dt = a.critical_dt(206e9, 0.3, 7850.0, 0.8)
+    for n in (37, 17, 31, 16, 2):
+        a.run(n, dt=dt, **params)
+        for _ in range(n):
+            b.run(1, dt=dt, **params)
+        assert np.array_equal(a.state(), b.state()) and np.array_equal(a.energy(), b.energy())
+    assert (a.state()[:, 12:120:15] > 0).sum() > 100, "the case must yield"
+    for x, y in zip(a.readback(), b.readback()):
+        assert np.array_equal(x, y)
+    assert a.stats() == b.stats()
