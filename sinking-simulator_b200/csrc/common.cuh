@@ -102,13 +102,13 @@ inline bool launch_cluster(void (*kernel)(Params...), int blocks, int threads, s
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
-        cudaGetLastError();
-        return false;
-    }
-    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...) == cudaSuccess;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kClusterSmem) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0 &&
+        cudaLaunchKernelEx(&cfg, kernel, Params(args)...) == cudaSuccess)
+        return true;
+    cudaGetLastError();  // the caller takes another way: no error is left for its checks
+    return false;
 }
 
 // Deterministic block sum in double: shuffle tree inside each warp, then warp 0 adds

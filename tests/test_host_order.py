@@ -88,3 +88,15 @@ def test_shell_step_after_a_graph_waits_for_it(fake, fibres):
         s.run(n, dt=1e-7)
         assert fake.lib.fake_early_after_graph() == 0
     s.close()
+
+
+@pytest.mark.parametrize("mode", ["ref32", "f32", "f32k", "f64"])
+def test_refused_cluster_launch_leaves_no_error(fake, mode):
+    """Where the launch of a small mesh's cluster is refused, the run takes two kernels a step
+    and succeeds."""
+    pos, idx, kw = tet_case(fake, mode, mode == "ref32")
+    s = fake.TetSolver(pos, idx, **kw)
+    fake.lib.fake_refuse_clusters(1)
+    s.run(200, dt=1e-6)
+    assert s.launches == 400 and fake.lib.fake_last_error() == 0
+    s.close()
