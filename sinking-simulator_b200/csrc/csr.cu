@@ -110,7 +110,9 @@ cudaError_t build_runs_device(const uint32_t* offset, const uint32_t* entry, lon
         err = cudaGetLastError();
     }
     if (span) cudaFreeAsync(span, stream);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(stream);
+    // on a failure too: the caller then frees arrays that queued kernels use
+    const cudaError_t end = cudaStreamSynchronize(stream);
+    if (err == cudaSuccess) err = end;
     *slots = count;
     return err;
 }

@@ -100,3 +100,15 @@ def test_refused_cluster_launch_leaves_no_error(fake, mode):
     s.run(200, dt=1e-6)
     assert s.launches == 400 and fake.lib.fake_last_error() == 0
     s.close()
+
+
+@pytest.mark.parametrize("mode", ["f32k", "f64"])
+def test_failed_create_frees_nothing_that_kernels_still_use(fake, mode):
+    """With no memory for the slot runs' scratch, create fails while its adjacency kernels are
+    still in flight: they are waited for before their arrays go back to the device's pool."""
+    pos, idx, kw = tet_case(fake, mode, False)
+    fake.lib.fake_fail_malloc(3)  # the two of the adjacency, then the runs'
+    with pytest.raises(fake.FemStepError) as e:
+        fake.TetSolver(pos, idx, **kw)
+    assert e.value.code == fake.ENOMEM
+    assert fake.lib.fake_freed_in_flight() == 0
