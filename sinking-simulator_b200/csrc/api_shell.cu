@@ -642,11 +642,12 @@ int femstep_shell_run(femstep_shell* s, int substeps, const femstep_shell_params
 int femstep_shell_readback(femstep_shell* s, double* position, double* velocity) {
     if (!s) return fail(s, FEMSTEP_EINVAL, "null solver");
     const size_t n3 = s->nodes * 3;
-    if (n3 >= kReadParallel && (position || velocity) &&
-        (s->pinned_slices || cudaHostAlloc((void**)&s->pinned_slices, kReadWorkers * 2 * kReadSlice * sizeof(float),
-                                           cudaHostAllocPortable) == cudaSuccess))
-        return read_slices(s, position, velocity);
-    cudaGetLastError();
+    if (n3 >= kReadParallel && (position || velocity)) {
+        if (s->pinned_slices || cudaHostAlloc((void**)&s->pinned_slices, kReadWorkers * 2 * kReadSlice * sizeof(float),
+                                              cudaHostAllocPortable) == cudaSuccess)
+            return read_slices(s, position, velocity);
+        cudaGetLastError();  // no pinned memory: the serial way
+    }
     std::vector<float> buf(n3);
     int rc = FEMSTEP_OK;
     if (position) {

@@ -112,3 +112,12 @@ def test_failed_create_frees_nothing_that_kernels_still_use(fake, mode):
         fake.TetSolver(pos, idx, **kw)
     assert e.value.code == fake.ENOMEM
     assert fake.lib.fake_freed_in_flight() == 0
+
+
+def test_small_readback_leaves_another_error_alone(fake):
+    """An error that another call of this thread has left pending is not this one's to clear."""
+    s = shell_zone(fake, 3, 3)
+    fake.lib.fake_set_last_error(1)
+    s.readback()
+    assert fake.lib.fake_last_error() == 1
+    s.close()
