@@ -281,3 +281,26 @@ def test_cluster_run_is_the_steps_to_the_bit(fem, mode, cells):
     assert np.array_equal(a.plastic(), b.plastic()) and np.array_equal(a.energy(), b.energy())
     if mode != "ref32" and nx > 10 and tip.any():
         assert (a.plastic()[:, 6] > 0).any(), "the case must yield"
+
+
+@pytest.mark.parametrize("cells", [(7, 3, 1), (16, 4, 1), (43, 1, 1), (13, 5, 2)])
+@pytest.mark.parametrize("pull", [2e4, 2e7])
+def test_f64_two_kernel_step_at_block_edges_and_large_rotations(fem, port, cells, pull):
+    """The same meshes and loads in runs too short for a cluster: two kernels a step, as every
+    large mesh has them, bit-identical to the FP64 oracle."""
+    nx, ny, nz = cells
+    pos, idx = fem.box_tet_mesh(0.1 * nx, 0.1 * ny, 0.1 * nz, nx, ny, nz)
+    fixed = (pos[0::3] < 1e-6).astype(np.uint32)
+    tip = pos[0::3] > 0.1 * nx - 1e-6
+    fext = np.zeros(pos.size)
+    fext[2::3][tip] = -pull * ny * nz / tip.sum()
+    ref = O.TetMesh64(port, pos, idx, fixed, fext)
+    dt = 0.5 * port.tet64_critical_dt(C.byref(ref._s), 210e9, 0.3, 7850.0, 0.9)
+    ref.step(O.tet64_params(dt=dt, ramp_steps=100), 400)
+    g = fem.TetSolver(pos, idx, mode="f64", fixed=fixed, external_force=fext, density=7850.0)
+    for _ in range(4):
+        g.run(100, dt=dt, ramp_steps=100)
+        assert g.launches == 200, "two kernels a step"
+    p, v = g.readback64()
+    assert np.array_equal(p, ref.position) and np.array_equal(v, ref.velocity)
+    assert np.array_equal(g.plastic().reshape(-1), ref.plastic)
