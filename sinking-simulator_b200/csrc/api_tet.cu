@@ -161,32 +161,52 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         for (size_t n = 0; n < N; ++n) fixed[n] = m.fixed[n] ? 1 : 0;
     const uint32_t* index = A.upload(m.index, T * 4);
     const float* pos32 = A.upload(m.position, N * 3);
-    uint2* run = A.alloc<uint2>(N);
-    uint32_t* slot = A.alloc<uint32_t>(T * 4);
-    long long slots = 0;
+    // What the set-up kernels write and what only they need, in two allocations besides the
+    // two widest arrays: each is a round trip to the driver, and a small mesh's create is little
+    // else (360 tets FP32: 308 us with one an array, 248 so; with the widest among them 43,200
+    // tets took 480 us for 465).
+    const bool wide = mode == FEMSTEP_TET_J2_F64;
+    size_t bytes = 0;
+    const auto place = [&bytes](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) & ~size_t(255);
+        return at;
+    };
+    const auto at = [](char* base, size_t offset) -> void* { return base + offset; };
+    const size_t run_at = place(N * sizeof(uint2)), slot_at = place(T * 4 * sizeof(uint32_t)),
+                 vol64_at = place(T * sizeof(double)), mass64_at = place(N * sizeof(double)), wide_end = bytes,
+                 vol32_at = place(T * sizeof(float)), mass32_at = place(N * sizeof(float)),
+                 inv_mass32_at = place(N * sizeof(float));
+    char* kept = A.alloc<char>(wide ? wide_end : bytes);
+    uint2* run = static_cast<uint2*>(at(kept, run_at));
+    uint32_t* slot = static_cast<uint32_t*>(at(kept, slot_at));
     // the FP64 rest state: Dm^-1 (SoA) and volumes per tet, lumped masses per node
     double* inv64 = A.alloc<double>(T * 9);
-    double* vol64 = A.alloc<double>(T);
-    double* mass64 = A.alloc<double>(N);
+    double* vol64 = static_cast<double*>(at(kept, vol64_at));
+    double* mass64 = static_cast<double*>(at(kept, mass64_at));
+    float* inv32 = wide ? nullptr : A.alloc<float>(T * 9);
     if (!A.ok()) {
         const int code = A.status() == cudaErrorMemoryAllocation ? FEMSTEP_ENOMEM : FEMSTEP_ECUDA;
         fail(s, code, std::string("device upload failed: ") + cudaGetErrorString(A.status()));
         femstep_tet_destroy(s);
         return code;
     }
-    uint32_t *entry = nullptr, *offset = nullptr;
-    double* quarter = nullptr;
-    rc = check(s, fs::device_alloc((void**)&entry, T * 4 * sizeof(uint32_t)), "alloc");
-    if (!rc) rc = check(s, fs::device_alloc((void**)&offset, (N + 1) * sizeof(uint32_t)), "alloc");
-    if (!rc) rc = check(s, fs::device_alloc((void**)&quarter, T * sizeof(double)), "alloc");
-    if (!rc) rc = check(s, fs::build_csr_device(index, (long long)T * 4, (long long)N, offset, slot, s->stream, entry),
+    bytes = 0;
+    const size_t entry_at = place(T * 4 * sizeof(uint32_t)), offset_at = place((N + 1) * sizeof(uint32_t)),
+                 quarter_at = place(T * sizeof(double)), count_at = place(sizeof(uint32_t));
+    char* scratch = nullptr;
+    rc = check(s, fs::device_alloc((void**)&scratch, bytes), "alloc");
+    uint32_t *entry = static_cast<uint32_t*>(at(scratch, entry_at)), *offset = static_cast<uint32_t*>(at(scratch, offset_at));
+    double* quarter = static_cast<double*>(at(scratch, quarter_at));
+    uint32_t* count = static_cast<uint32_t*>(at(scratch, count_at));
+    if (!rc) rc = check(s, fs::build_csr_device(index, (long long)T * 4, (long long)N, offset, nullptr, s->stream, entry),
                         "adjacency");
     if (!rc) {
         fs::launch_tet_rest64(pos32, index, (long long)T, m.density, inv64, vol64, quarter, s->stream);
         fs::launch_tet_mass64(offset, entry, (long long)N, quarter, mass64, s->stream);
         rc = check(s, cudaGetLastError(), "rest state");
     }
-    if (!rc) rc = check(s, fs::build_runs_device(offset, entry, (long long)T * 4, (long long)N, run, slot, &slots, s->stream),
+    if (!rc) rc = check(s, fs::build_runs_device(offset, entry, (long long)T * 4, (long long)N, run, slot, count, s->stream),
                         "slot runs");
 
     auto common = [&](auto& d) {
@@ -196,7 +216,6 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         d.slot = reinterpret_cast<const uint4*>(slot);
         d.fixed = A.upload(fixed.data(), N);
         d.run = run;
-        d.slot_count = slots;
         // the step counter, the energy partials and the reductions' output, in one piece
         double* zero = A.zeros<double>(8 + 2 + 2 * (size_t)s->eblocks + 3 * (size_t)s->nblocks);
         s->d_out = zero;
@@ -207,7 +226,7 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         d.n_kin = d.n_work + s->nblocks;
         d.n_grav = d.n_kin + s->nblocks;
     };
-    if (!rc && mode == FEMSTEP_TET_J2_F64) {
+    if (!rc && wide) {
         TetDevice<double>& d = s->d64;
         common(d);
         double* pos = A.alloc<double>(N * 3);
@@ -224,29 +243,31 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         d.rest_vol = vol64;
         d.plastic = A.zeros<double>(T * 7);
         if (m.external_force) d.ext = A.upload(m.external_force, N * 3);
-        d.slots = A.alloc<double>((size_t)slots * 3);
     } else if (!rc) {
         TetDevice<float>& d = s->d32;
+        float* vol32 = static_cast<float*>(at(kept, vol32_at));
+        float* mass32 = static_cast<float*>(at(kept, mass32_at));
+        float* inv_mass32 = static_cast<float*>(at(kept, inv_mass32_at));
+        fs::launch_tet_rest_f32(inv64, vol64, (long long)T, mass64, (long long)N, inv32, vol32, mass32, inv_mass32, s->stream);
         common(d);
         d.velocity = m.velocity ? A.upload(m.velocity, N * 3) : A.zeros<float>(N * 3);
-        d.slots = A.alloc<float>((size_t)slots * 4);  // a padded float4 per corner
         s->rest.assign(m.position, m.position + N * 3);
         d.rest = pos32;
-        d.disp = A.zeros<float>(N * 4);
-        if (mode == FEMSTEP_TET_J2_F32K) d.disp_c = A.zeros<float>(N * 4);
-        float* inv32 = A.alloc<float>(T * 9);
-        float* vol32 = A.alloc<float>(T);
-        float* mass32 = A.alloc<float>(N);
-        float* inv_mass32 = A.alloc<float>(N);
-        if (A.ok())
-            fs::launch_tet_rest_f32(inv64, vol64, (long long)T, mass64, (long long)N, inv32, vol32, mass32, inv_mass32,
-                                    s->stream);
+        const bool comp = mode == FEMSTEP_TET_J2_F32K;
+        bytes = 0;
+        const size_t disp_at = place(N * 4 * sizeof(float)), plastic_at = place(T * 7 * sizeof(float)), plain_end = bytes,
+                     disp_c_at = place(N * 4 * sizeof(float)), plastic_c_at = place(T * 7 * sizeof(float));
+        char* zero = A.zeros<char>(comp ? bytes : plain_end);
+        d.disp = static_cast<float*>(at(zero, disp_at));
+        d.plastic = static_cast<float*>(at(zero, plastic_at));
+        if (comp) {
+            d.disp_c = static_cast<float*>(at(zero, disp_c_at));
+            d.plastic_c = static_cast<float*>(at(zero, plastic_c_at));
+        }
         d.rest_inv = inv32;
         d.rest_vol = vol32;
         d.mass = mass32;
         d.inv_mass = inv_mass32;
-        d.plastic = A.zeros<float>(T * 7);
-        if (mode == FEMSTEP_TET_J2_F32K) d.plastic_c = A.zeros<float>(T * 7);
         if (m.external_force) {
             std::vector<float> ext(N * 3);
             for (size_t i = 0; i < N * 3; ++i) ext[i] = (float)m.external_force[i];
@@ -254,11 +275,21 @@ int create_on_device(const femstep_tet_mesh& m, int mode, femstep_tet** out) {
         }
         s->inv64 = inv64;
     }
-    if (!rc) rc = check(s, cudaStreamSynchronize(s->stream), "set-up");
+    // The kernels have run beside the uploads; only the slots wait for their count.  (Waited for
+    // on a failure too: queued kernels use the scratch.)
+    uint32_t slots = 0;
+    if (!rc) rc = check(s, cudaMemcpyAsync(&slots, count, sizeof(slots), cudaMemcpyDeviceToHost, s->stream), "slot runs");
+    const cudaError_t end = cudaStreamSynchronize(s->stream);
+    if (!rc) rc = check(s, end, "set-up");
+    if (!rc && wide) {
+        s->d64.slot_count = slots;
+        s->d64.slots = A.alloc<double>((size_t)slots * 3);
+    } else if (!rc) {
+        s->d32.slot_count = slots;
+        s->d32.slots = A.alloc<float>((size_t)slots * 4);  // a padded float4 per corner
+    }
     if (!rc) rc = check(s, cudaStreamSynchronize(cudaStreamLegacy), "upload");  // the last uploads, before any step
-    fs::device_free(entry);
-    fs::device_free(offset);
-    fs::device_free(quarter);
+    fs::device_free(scratch);
     if (!rc && !A.ok()) {
         const int code = A.status() == cudaErrorMemoryAllocation ? FEMSTEP_ENOMEM : FEMSTEP_ECUDA;
         rc = fail(s, code, std::string("device upload failed: ") + cudaGetErrorString(A.status()));
@@ -306,15 +337,28 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
     } else {
         fs::build_csr(N, T, 4, m.index, offset, entry);
     }
-    {
-        std::vector<bool> seen(T * 4, false);
-        for (size_t n = 0; n < N; ++n)
-            for (uint32_t k = offset[n]; k < offset[n + 1]; ++k) {
-                const uint32_t e = entry[k];
-                if (e >= T * 4 || m.index[e] != n || seen[e])
+    std::vector<uint2> run(N);
+    std::vector<uint32_t> slot(T * 4, 0xffffffffu);
+    long long slots = 0;
+    const bool allow = (long long)T * 4 < fs::kRunStridedMost;
+    for (size_t n0 = 0; n0 < N; n0 += 32) {
+        const size_t n1 = std::min(N, n0 + 32);
+        uint32_t longest = 0;
+        for (size_t n = n0; n < n1; ++n) longest = std::max(longest, offset[n + 1] - offset[n]);
+        const uint32_t sum = offset[n1] - offset[n0];
+        const bool strided = fs::run_strided(longest, sum, allow);
+        for (size_t n = n0; n < n1; ++n) {
+            const uint32_t count = offset[n + 1] - offset[n], step = strided ? 32u : 1u;
+            const uint32_t start = (uint32_t)slots + (strided ? (uint32_t)(n - n0) : offset[n] - offset[n0]);
+            run[n] = make_uint2(start, count | (strided ? fs::kRunStrided : 0u));
+            for (uint32_t k = 0; k < count; ++k) {
+                const uint32_t e = entry[offset[n] + k];
+                if (e >= T * 4 || m.index[e] != n || slot[e] != 0xffffffffu)
                     return fail(nullptr, FEMSTEP_EINVAL, "adjacency is not the node-to-corner map of this mesh");
-                seen[e] = true;
+                slot[e] = start + k * step;
             }
+        }
+        slots += strided ? 32u * longest : sum;
     }
     // The mesh is checked before the device, so a bad mesh is reported as such on any
     // machine; a good one on a machine with no GPU is a skip.
@@ -342,36 +386,13 @@ int femstep_tet_create(const femstep_tet_mesh* mesh, int mode, femstep_tet** out
     std::vector<double> inv64, vol64, mass64;
     if (mode != FEMSTEP_TET_REF32) rest_state64(m, inv64, vol64, mass64);
 
-    uint2* run = A.alloc<uint2>(N);
-    uint32_t* slot = A.alloc<uint32_t>(T * 4);
-    long long slots = 0;
-    {
-        uint32_t *doffset = nullptr, *dentry = nullptr;
-        rc = check(s, fs::device_alloc((void**)&doffset, (N + 1) * sizeof(uint32_t)), "alloc");
-        if (!rc) rc = check(s, fs::device_alloc((void**)&dentry, T * 4 * sizeof(uint32_t)), "alloc");
-        if (!rc) rc = check(s, cudaMemcpy(doffset, offset.data(), (N + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
-        if (!rc) rc = check(s, cudaMemcpy(dentry, entry.data(), T * 4 * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
-        // (a copy from pageable memory may return before it has landed, and the solver's
-        // stream does not wait for the legacy one)
-        if (!rc) rc = check(s, cudaStreamSynchronize(cudaStreamLegacy), "upload");
-        if (!rc && A.ok())
-            rc = check(s, fs::build_runs_device(doffset, dentry, (long long)T * 4, (long long)N, run, slot, &slots, s->stream),
-                       "slot runs");
-        fs::device_free(doffset);
-        fs::device_free(dentry);
-        if (rc) {
-            femstep_tet_destroy(s);
-            return rc;
-        }
-    }
-
     auto common = [&](auto& d) {
         d.nodes = (long long)N;
         d.tets = (long long)T;
         d.index = (const uint4*)A.upload(m.index, T * 4);
-        d.slot = reinterpret_cast<const uint4*>(slot);
+        d.slot = (const uint4*)A.upload(slot.data(), T * 4);
         d.fixed = A.upload(fixed.data(), N);
-        d.run = run;
+        d.run = A.upload(run.data(), N);
         d.slot_count = slots;
         // the step counter, the energy partials and the reductions' output, in one piece
         double* zero = A.zeros<double>(8 + 2 + 2 * (size_t)s->eblocks + 3 * (size_t)s->nblocks);

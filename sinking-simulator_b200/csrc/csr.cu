@@ -53,12 +53,8 @@ __global__ void csr_slots(const uint32_t* entry, const uint32_t* counted, uint32
         slot[entry[k]] = base + (uint32_t)k;
 }
 
-// The strided layout of the nodes' slot runs (build_runs_device): a warp takes a group of
-// 32 consecutive nodes.
-__device__ __forceinline__ bool run_strided(uint32_t longest, uint32_t sum, bool allow) {
-    return allow && (unsigned long long)longest * 32 <= 2ull * sum;
-}
-
+// The layout of the nodes' slot runs (build_runs_device): a warp takes a group of 32
+// consecutive nodes.
 __global__ void run_spans(const uint32_t* offset, long long nodes, bool allow, uint32_t* span) {
     const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t count = n < nodes ? offset[n + 1] - offset[n] : 0u;
@@ -89,13 +85,12 @@ __global__ void csr_add_base(uint32_t* offset, long long n, uint32_t base) {
 }  // namespace
 
 cudaError_t build_runs_device(const uint32_t* offset, const uint32_t* entry, long long total, long long nodes, uint2* run,
-                              uint32_t* slot, long long* slots, cudaStream_t stream) {
+                              uint32_t* slot, uint32_t* slots, cudaStream_t stream) {
     const int groups = blocks_for(nodes, 32) + 1;
-    const bool allow = total < (1ll << 30);  // padded runs at most double the slots: 32-bit ids hold them
+    const bool allow = total < kRunStridedMost;
     uint32_t* span = nullptr;
     void* temp = nullptr;
     size_t temp_bytes = 0;
-    uint32_t count = 0;
     cudaError_t err = cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, span, span, groups, stream);
     const size_t scan_at = ((size_t)groups * 2 * sizeof(uint32_t) + 255) & ~size_t(255);
     if (err == cudaSuccess) err = cudaMallocAsync(&span, scan_at + temp_bytes, stream);
@@ -106,14 +101,10 @@ cudaError_t build_runs_device(const uint32_t* offset, const uint32_t* entry, lon
     }
     if (err == cudaSuccess) {
         run_fill<<<blocks_for(nodes, 256), 256, 0, stream>>>(offset, entry, nodes, allow, span + groups, run, slot);
-        cudaMemcpyAsync(&count, span + 2 * groups - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream);
-        err = cudaGetLastError();
+        err = cudaMemcpyAsync(slots, span + 2 * groups - 1, sizeof(uint32_t), cudaMemcpyDeviceToDevice, stream);
+        if (err == cudaSuccess) err = cudaGetLastError();
     }
     if (span) cudaFreeAsync(span, stream);
-    // on a failure too: the caller then frees arrays that queued kernels use
-    const cudaError_t end = cudaStreamSynchronize(stream);
-    if (err == cudaSuccess) err = end;
-    *slots = count;
     return err;
 }
 
@@ -139,7 +130,7 @@ cudaError_t build_csr_device(const uint32_t* index, long long total, long long n
         const int grid = 148 * 8;
         csr_scatter<<<grid, 256, 0, stream>>>(index, total, nodes, count, entry);
         csr_sort_runs<<<blocks_for(nodes, 256), 256, 0, stream>>>(offset, nodes, entry);
-        csr_slots<<<grid, 256, 0, stream>>>(entry, offset + nodes, slot, base);
+        if (slot) csr_slots<<<grid, 256, 0, stream>>>(entry, offset + nodes, slot, base);
         if (base) csr_add_base<<<grid, 256, 0, stream>>>(offset, nodes + 1, base);
         err = cudaGetLastError();
     }

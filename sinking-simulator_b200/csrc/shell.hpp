@@ -194,7 +194,7 @@ struct ShellSetupArgs {
 };
 void launch_shell_setup(const ShellSetupArgs& a, cudaStream_t stream);
 // The node -> corner adjacency in element order and the corner -> CSR slot map, on the
-// device (csr.cu): offset [nodes + 1], slot [total]; index values must be < nodes.
+// device (csr.cu): offset [nodes + 1], slot [total] (may be null); index values must be < nodes.
 // `entry_out` [total], if given, receives the adjacency entries themselves; `base` is
 // added to every offset and slot (a CSR placed at that position of a larger one).
 cudaError_t build_csr_device(const uint32_t* index, long long total, long long nodes, uint32_t* offset, uint32_t* slot,

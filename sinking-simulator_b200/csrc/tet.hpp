@@ -89,6 +89,14 @@ struct TetParams {
 // `parts`: kElementPart | kNodePart (a whole step), or one of them alone (profiling).
 constexpr uint32_t kRunStrided = 0x80000000u;  // in TetDevice::run's length
 
+// Whether the runs of a group of 32 consecutive nodes lie strided, 32 x `longest` slots, or
+// one after the other, `sum` slots.  `allow`: fewer corners than kRunStridedMost, of which
+// runs padded to at most twice the slots still have 32-bit ids.
+constexpr long long kRunStridedMost = 1ll << 30;
+__host__ __device__ __forceinline__ bool run_strided(uint32_t longest, uint32_t sum, bool allow) {
+    return allow && (unsigned long long)longest * 32 <= 2ull * sum;
+}
+
 // A node's run of slots: slot k at start + k * step.
 struct SlotRun {
     uint32_t start, count, step;
@@ -113,9 +121,9 @@ __device__ __forceinline__ void for_run(const SlotRun& r, Load load, Add add) {
 }
 
 // The runs of a CSR (adjacency offsets and entries): run [nodes], slot [total] and the
-// number of slots, read back (waits for the stream).
+// number of slots, all on the device (queued on `stream`, not waited for).
 cudaError_t build_runs_device(const uint32_t* offset, const uint32_t* entry, long long total, long long nodes, uint2* run,
-                              uint32_t* slot, long long* slots, cudaStream_t stream);
+                              uint32_t* slot, uint32_t* slots, cudaStream_t stream);
 
 // Threads per block of the single-mesh node kernels: few, so that a small mesh's nodes
 // spread over the SMs.

@@ -23,6 +23,7 @@ int g_malloc_fails_at = 0;       // the n-th allocation on a handle's own stream
 bool g_capturing = false;
 bool g_after_graph = false;      // the stream's last work is a graph launch
 int g_early_after_graph = 0;     // programmatic launches right after one
+int g_calls = 0;                 // launches, allocations, copies, memsets and waits
 
 cudaError_t result(cudaError_t e) {
     if (e != cudaSuccess) g_last = e;
@@ -30,6 +31,7 @@ cudaError_t result(cudaError_t e) {
 }
 
 void launched(bool early) {
+    ++g_calls;
     if (g_capturing) return;
     if (g_pending) ++g_unordered;
     if (g_after_graph && early) ++g_early_after_graph;
@@ -45,6 +47,7 @@ int fake_pending() { return g_pending; }
 int fake_unordered() { return g_unordered; }
 int fake_freed_in_flight() { return g_freed_in_flight; }
 int fake_early_after_graph() { return g_early_after_graph; }
+int fake_calls() { return g_calls; }
 int fake_last_error() { return (int)g_last; }
 void fake_set_last_error(int e) { g_last = (cudaError_t)e; }
 void fake_refuse_clusters(int on) { g_refuse_clusters = on; }
@@ -52,7 +55,7 @@ void fake_fail_malloc(int n) { g_malloc_fails_at = n; }
 void fake_reset() {
     g_last = cudaSuccess;
     g_pending = g_in_flight = g_unordered = g_freed_in_flight = g_refuse_clusters = g_malloc_fails_at = 0;
-    g_early_after_graph = 0;
+    g_early_after_graph = g_calls = 0;
     g_capturing = g_after_graph = false;
 }
 
@@ -90,12 +93,14 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* cfg, const void*, void
 
 // ---- memory ----
 cudaError_t cudaMallocAsync(void** p, size_t bytes, cudaStream_t stream) {
+    ++g_calls;
     if (stream != cudaStreamLegacy && g_malloc_fails_at && --g_malloc_fails_at == 0) return result(cudaErrorMemoryAllocation);
     *p = std::aligned_alloc(256, (bytes + 255) / 256 * 256 + 256);
     std::memset(*p, 0, (bytes + 255) / 256 * 256 + 256);
     return cudaSuccess;
 }
 cudaError_t cudaFreeAsync(void* p, cudaStream_t stream) {
+    ++g_calls;
     if (stream == cudaStreamLegacy && g_in_flight) ++g_freed_in_flight;
     std::free(p);
     return cudaSuccess;
@@ -109,20 +114,24 @@ cudaError_t cudaFreeHost(void* p) {
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* dst, const void* src, size_t bytes, cudaMemcpyKind kind) {
+    ++g_calls;
     std::memcpy(dst, src, bytes);
     g_pending = kind == cudaMemcpyHostToDevice ? g_pending + 1 : 0;
     return cudaSuccess;
 }
 cudaError_t cudaMemset(void* dst, int value, size_t bytes) {
+    ++g_calls;
     std::memset(dst, value, bytes);
     ++g_pending;
     return cudaSuccess;
 }
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t bytes, cudaMemcpyKind, cudaStream_t) {
+    ++g_calls;
     std::memcpy(dst, src, bytes);
     return cudaSuccess;
 }
 cudaError_t cudaMemsetAsync(void* dst, int value, size_t bytes, cudaStream_t) {
+    ++g_calls;
     std::memset(dst, value, bytes);
     return cudaSuccess;
 }
@@ -137,6 +146,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) {
     return cudaSuccess;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
+    ++g_calls;
     (s == cudaStreamLegacy ? g_pending : g_in_flight) = 0;
     return cudaSuccess;
 }

@@ -71,6 +71,18 @@ def test_tet_uploads_land_before_the_solver_reads_them(fake, mode, adjacency, lo
     s.close()
 
 
+@pytest.mark.parametrize("mode,adjacency,most", [("ref32", True, 51), ("f32k", True, 70), ("f32k", False, 80),
+                                                 ("f64", True, 60), ("f64", False, 80)])
+def test_tet_create_makes_few_calls(fake, mode, adjacency, most):
+    """Every allocation, copy, wait and launch of a create is some 3 us of a small mesh's 250:
+    what can share one does."""
+    pos, idx, kw = tet_case(fake, mode, adjacency)
+    fake.lib.fake_reset()
+    s = fake.TetSolver(pos, idx, **kw)
+    assert fake.lib.fake_calls() <= most
+    s.close()
+
+
 def shell_zone(fem, nx, ny):
     rest, index, pinned, load = fem.stiffened_panel(nx=nx, ny=ny, lx=0.01 * nx, ly=0.01 * ny, thickness=0.008,
                                                     stiffeners=0, imperfection=2e-4, peak_pressure=4e7, radius=10.0)
