@@ -555,25 +555,25 @@ __global__ void f32_positions(const float4* disp, const float4* disp_c, const fl
     out[n * 3 + 2] = (Out)((double)rest[n * 3 + 2] + ((double)u.z - (double)c.z));
 }
 
-// They go to the caller formed on the device, in one copy without padding; where the device
-// has no room for them, they are formed here from the two padded arrays (88,641 nodes:
-// positions and velocities in 1.9 ms so, 1.0 ms from the device).
+// They go to the caller formed on the device, in one copy without padding, through the force
+// slots, which hold nothing between steps (88,641 nodes: positions and velocities in 1.9 ms from
+// the two padded arrays, 1.0 ms from the device; taking memory for it instead cost a small mesh
+// 10 of its 40 us).  A mesh of fewer slots than that, all but a few of its nodes in no tet,
+// has them formed here.
 template <class Out>
 int read_positions(femstep_tet* s, Out* position) {
     const size_t n3 = s->nodes * 3;
-    void* out = nullptr;
-    if (fs::device_alloc(&out, n3 * sizeof(Out)) == cudaSuccess) {  // (which waits for the legacy stream)
+    if (n3 * sizeof(Out) <= (size_t)s->d32.slot_count * sizeof(float4)) {
+        Out* out = reinterpret_cast<Out*>(s->d32.slots);
         f32_positions<Out><<<fs::blocks_for((long long)s->nodes, 256), 256, 0, s->stream>>>(
             reinterpret_cast<const float4*>(s->d32.disp), reinterpret_cast<const float4*>(s->d32.disp_c), s->d32.rest,
-            (long long)s->nodes, static_cast<Out*>(out));
+            (long long)s->nodes, out);
         int rc = check(s, cudaGetLastError(), "readback");
         if (!rc)
             rc = check(s, cudaMemcpyAsync(position, out, n3 * sizeof(Out), cudaMemcpyDeviceToHost, s->stream), "readback");
         if (!rc) rc = check(s, cudaStreamSynchronize(s->stream), "readback");
-        fs::device_free(out);
         return rc;
     }
-    cudaGetLastError();
     std::vector<double> u;
     const int rc = displacement(s, u);
     for (size_t i = 0; i < n3 && !rc; ++i) position[i] = (Out)((double)s->rest[i] + u[i]);

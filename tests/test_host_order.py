@@ -133,3 +133,16 @@ def test_small_readback_leaves_another_error_alone(fake):
     s.readback()
     assert fake.lib.fake_last_error() == 1
     s.close()
+
+
+@pytest.mark.parametrize("mode", ["f32", "f32k"])
+def test_tet_readback_takes_no_device_memory(fake, mode):
+    """The positions formed on the device go through memory that the solver has: a launch, a copy
+    and a wait for them, and the velocities' copy."""
+    pos, idx, kw = tet_case(fake, mode, False)
+    s = fake.TetSolver(pos, idx, **kw)
+    for read in (s.readback, s.readback64):
+        fake.lib.fake_reset()
+        read()
+        assert fake.lib.fake_calls() <= 4
+    s.close()

@@ -304,3 +304,28 @@ def test_f64_two_kernel_step_at_block_edges_and_large_rotations(fem, port, cells
     p, v = g.readback64()
     assert np.array_equal(p, ref.position) and np.array_equal(v, ref.velocity)
     assert np.array_equal(g.plastic().reshape(-1), ref.plastic)
+
+
+@pytest.mark.parametrize("mode", ["f32", "f32k"])
+@pytest.mark.parametrize("spare", [0, 11, 12, 400])
+def test_readback_between_runs_changes_nothing(fem, mode, spare):
+    """The FP32 modes' positions are formed on the device in the force slots, or on the host
+    where the nodes in no tet (one tet of four nodes and 4 slots, up to 404 nodes) outnumber
+    them: the same positions either way, and steps after a readback are those without one."""
+    pos = np.concatenate([[0, 0, 0, 1, 0, 0, 0, 1, 0, 0, 0, 1], 3.0 + 0.01 * np.arange(3 * spare)]).astype(np.float32)
+    idx = np.array([0, 1, 2, 3], np.uint32)
+    fixed = np.zeros(pos.size // 3, np.uint32)
+    fixed[0] = 1
+    ext = np.zeros(pos.size)
+    ext[3:6] = 1e5
+    a, b = (fem.TetSolver(pos, idx, mode=mode, fixed=fixed, external_force=ext, density=7850.0) for _ in range(2))
+    run = dict(dt=2e-5, ramp_steps=10)
+    for n in (7, 40, 3):
+        a.run(n, **run)
+        b.run(n, **run)
+        p, v = a.readback64()
+        q, w = a.readback()
+        assert np.array_equal(p.astype(np.float32), q) and np.array_equal(v, w)
+    assert np.abs(p[:12] - pos[:12]).max() > 1e-6
+    pb, vb = b.readback64()
+    assert np.array_equal(p, pb) and np.array_equal(v, vb) and np.array_equal(a.energy(), b.energy())
