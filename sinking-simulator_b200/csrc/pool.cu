@@ -546,46 +546,12 @@ __global__ void pool_admit_tets(PoolDevice d, const PoolAdmit* adm, int G, long 
     }
 }
 
-// Per node of the group (and each mesh's spare slot): its lumped mass from the tets'
-// quarters, then displacement, compensation and velocity at rest (the velocity rows
-// held the staged positions until now).
-__global__ void pool_admit_nodes(PoolDevice d, const PoolAdmit* adm, int G, long long nodes) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nodes; k += stride) {
-        const PoolAdmit& a = adm[admit_of<&PoolAdmit::node_first>(adm, G, k)];
-        const long long n = k - a.node_first;
-        rest_node(d, a.n0, a.N, n);
-        d.disp[a.n0 + n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        d.disp_c[a.n0 + n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        float* v = d.velocity + (size_t)(a.n0 + n) * 3;
-        v[0] = v[1] = v[2] = 0.0f;
-    }
-}
-
-// Per tet of a mesh that wants its step formed: the element bound from the stored
-// FP32 Dm^-1 (promoted to double), maximised per mesh.  A non-negative double orders
-// as its bit pattern, so the maximum is an integer atomicMax and exact.
-__global__ void pool_admit_omega(PoolDevice d, const PoolAdmit* adm, int G, long long tets,
-                                 unsigned long long* w2) {
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < tets; k += stride) {
-        const int g = admit_of<&PoolAdmit::tet_first>(adm, G, k);
-        const PoolAdmit& a = adm[g];
-        if (!a.want_dt) continue;
-        const long long t = a.t0 + (k - a.tet_first);
-        double gr[4][3];
-        for (int c = 0; c < 3; ++c)
-            for (int r = 0; r < 3; ++r) gr[c + 1][r] = (double)d.rest_inv[(size_t)(r * 3 + c) * d.tet_cap + t];
-        for (int r = 0; r < 3; ++r) gr[0][r] = -(gr[1][r] + gr[2][r] + gr[3][r]);
-        const double v = tet_omega2_one<true>(gr, a.lambda, a.mu, a.density);
-        atomicMax(w2 + g, (unsigned long long)__double_as_longlong(v > 0.0 ? v : 0.0));
-    }
-}
-
 // The slot map of the group's tets, from CSR places to the jagged ones (jagged_gather):
 // slot k of a node goes to its 32 nodes' first slot, past their first k slots each, by
-// its rank.  Last of the admission: the rest state's masses are summed over the CSR.
-__global__ void pool_jag(PoolDevice d, const PoolAdmit* adm, int G, long long tets) {
+// its rank.  In the launch after pool_admit_tets, which still puts the rest state's masses by
+// the CSR places; pool_admit_nodes sums them there without the map.  (A launch of its own cost
+// a mesh's admission 3 of 72 us.)
+__device__ __forceinline__ void pool_jag(const PoolDevice& d, const PoolAdmit* adm, int G, long long tets) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < tets; x += stride) {
         const PoolAdmit& a = adm[admit_of<&PoolAdmit::tet_first>(adm, G, x)];
@@ -608,6 +574,43 @@ __global__ void pool_jag(PoolDevice d, const PoolAdmit* adm, int G, long long te
             sl[c] = place;
         }
         d.slot[t] = make_uint4(sl[0], sl[1], sl[2], sl[3]);
+    }
+}
+
+// Per node of the group (and each mesh's spare slot): its lumped mass from the tets'
+// quarters, then displacement, compensation and velocity at rest (the velocity rows
+// held the staged positions until now).
+__global__ void pool_admit_nodes(PoolDevice d, const PoolAdmit* adm, int G, long long nodes, long long tets) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < nodes; k += stride) {
+        const PoolAdmit& a = adm[admit_of<&PoolAdmit::node_first>(adm, G, k)];
+        const long long n = k - a.node_first;
+        rest_node(d, a.n0, a.N, n);
+        d.disp[a.n0 + n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        d.disp_c[a.n0 + n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float* v = d.velocity + (size_t)(a.n0 + n) * 3;
+        v[0] = v[1] = v[2] = 0.0f;
+    }
+    pool_jag(d, adm, G, tets);
+}
+
+// Per tet of a mesh that wants its step formed: the element bound from the stored
+// FP32 Dm^-1 (promoted to double), maximised per mesh.  A non-negative double orders
+// as its bit pattern, so the maximum is an integer atomicMax and exact.
+__global__ void pool_admit_omega(PoolDevice d, const PoolAdmit* adm, int G, long long tets,
+                                 unsigned long long* w2) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < tets; k += stride) {
+        const int g = admit_of<&PoolAdmit::tet_first>(adm, G, k);
+        const PoolAdmit& a = adm[g];
+        if (!a.want_dt) continue;
+        const long long t = a.t0 + (k - a.tet_first);
+        double gr[4][3];
+        for (int c = 0; c < 3; ++c)
+            for (int r = 0; r < 3; ++r) gr[c + 1][r] = (double)d.rest_inv[(size_t)(r * 3 + c) * d.tet_cap + t];
+        for (int r = 0; r < 3; ++r) gr[0][r] = -(gr[1][r] + gr[2][r] + gr[3][r]);
+        const double v = tet_omega2_one<true>(gr, a.lambda, a.mu, a.density);
+        atomicMax(w2 + g, (unsigned long long)__double_as_longlong(v > 0.0 ? v : 0.0));
     }
 }
 
@@ -644,8 +647,7 @@ void launch_pool_admit(const PoolDevice& d, const PoolAdmit* adm, int G, long lo
     const int cap = sm_count() * 8;
     auto grid = [&](long long n) { return (int)std::max(1LL, std::min((long long)cap, (n + kBlock - 1) / kBlock)); };
     pool_admit_tets<<<grid(std::max(tets, parts)), kBlock, 0, stream>>>(d, adm, G, tets, parts);
-    pool_admit_nodes<<<grid(nodes), kBlock, 0, stream>>>(d, adm, G, nodes);
-    pool_jag<<<grid(tets), kBlock, 0, stream>>>(d, adm, G, tets);
+    pool_admit_nodes<<<grid(std::max(nodes, tets)), kBlock, 0, stream>>>(d, adm, G, nodes, tets);
     if (any_dt) {
         cudaMemsetAsync(w2, 0, (size_t)G * sizeof(unsigned long long), stream);
         pool_admit_omega<<<grid(tets), kBlock, 0, stream>>>(d, adm, G, tets, w2);

@@ -146,3 +146,16 @@ def test_tet_readback_takes_no_device_memory(fake, mode):
         read()
         assert fake.lib.fake_calls() <= 4
     s.close()
+
+
+def test_pool_admission_launches_no_more_than_it_needs(fake):
+    """A mesh's admission: its record and arrays, the adjacency, the rest state by tets and by
+    nodes."""
+    pos, idx = fake.box_tet_mesh(0.4, 0.1, 0.02, 4, 2, 2)
+    pool = fake.TetPool(20000, 8000, max_meshes=8, tile=128)
+    mesh = dict(position=pos, index=idx, external_force=np.ones(pos.size), dt=1e-8)
+    pool.admit_many([mesh], [5])
+    fake.lib.fake_reset()
+    pool.admit_many([mesh], [5])
+    assert fake.lib.fake_calls() <= 25
+    pool.close()
