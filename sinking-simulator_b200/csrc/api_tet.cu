@@ -556,14 +556,17 @@ __global__ void f32_positions(const float4* disp, const float4* disp_c, const fl
 }
 
 // They go to the caller formed on the device, in one copy without padding, through the force
-// slots, which hold nothing between steps (88,641 nodes: positions and velocities in 1.9 ms from
-// the two padded arrays, 1.0 ms from the device; taking memory for it instead cost a small mesh
-// 10 of its 40 us).  A mesh of fewer slots than that, all but a few of its nodes in no tet,
-// has them formed here.
+// slots, which hold nothing between steps; positions and velocities of 88,641 nodes take 1.0 ms
+// so and 1.9 ms formed here from the two padded arrays.  Formed here all the same: a mesh of
+// fewer slots than that, all but a few of its nodes in no tet; and a small one in the plain
+// mode, whose one padded array comes quicker than a kernel, a copy and a wait (132 nodes 29 us
+// for 36, 1,152 nodes 45 for 50, 8,577 nodes 109 for 84; of two arrays 132 nodes take 45).
+constexpr size_t kPlainHostNodes = 2048;
+
 template <class Out>
 int read_positions(femstep_tet* s, Out* position) {
     const size_t n3 = s->nodes * 3;
-    if (n3 * sizeof(Out) <= (size_t)s->d32.slot_count * sizeof(float4)) {
+    if ((s->d32.disp_c || s->nodes >= kPlainHostNodes) && n3 * sizeof(Out) <= (size_t)s->d32.slot_count * sizeof(float4)) {
         Out* out = reinterpret_cast<Out*>(s->d32.slots);
         f32_positions<Out><<<fs::blocks_for((long long)s->nodes, 256), 256, 0, s->stream>>>(
             reinterpret_cast<const float4*>(s->d32.disp), reinterpret_cast<const float4*>(s->d32.disp_c), s->d32.rest,
