@@ -160,3 +160,15 @@ def test_pool_admission_launches_no_more_than_it_needs(fake):
     pool.admit_many([mesh], [5])
     assert fake.lib.fake_calls() <= 25
     pool.close()
+
+
+def test_shell_create_makes_few_calls(fake):
+    """A zone whose groups are taken in an order asks for no memory of its own for it: it is
+    created with the calls of the smaller zones, which have none."""
+    calls = []
+    for nx, ny in ((88, 80), (90, 80)):  # 7,040 elements, one wave; 7,200
+        fake.lib.fake_reset()
+        s = shell_zone(fake, nx, ny)
+        calls.append(fake.lib.fake_calls())
+        s.close()
+    assert calls[0] == calls[1]

@@ -329,3 +329,24 @@ def test_readback_between_runs_changes_nothing(fem, mode, spare):
     assert np.abs(p[:12] - pos[:12]).max() > 1e-6
     pb, vb = b.readback64()
     assert np.array_equal(p, pb) and np.array_equal(v, vb) and np.array_equal(a.energy(), b.energy())
+
+
+@pytest.mark.parametrize("mode", ["f32", "f32k"])
+@pytest.mark.parametrize("cells", [(11, 13, 11), (15, 15, 7), (13, 13, 13)])
+def test_readback_between_runs_of_a_box(fem, mode, cells):
+    """The same for meshes of 2,016, 2,048 and 2,744 nodes, around the line under which the plain
+    mode forms its positions on the host."""
+    nx, ny, nz = cells
+    pos, idx = fem.box_tet_mesh(0.05 * nx, 0.05 * ny, 0.05 * nz, nx, ny, nz)
+    fixed = (pos[0::3] < 1e-6).astype(np.uint32)
+    a, b = (fem.TetSolver(pos, idx, mode=mode, fixed=fixed, density=7850.0) for _ in range(2))
+    run = dict(dt=2e-6, gravity=9.80665)
+    for n in (3, 40):
+        a.run(n, **run)
+        b.run(n, **run)
+        p, v = a.readback64()
+        q, w = a.readback()
+        assert np.array_equal(p.astype(np.float32), q) and np.array_equal(v, w)
+    assert np.abs(p - pos).max() > 1e-8
+    pb, vb = b.readback64()
+    assert np.array_equal(p, pb) and np.array_equal(v, vb) and np.array_equal(a.energy(), b.energy())
