@@ -114,7 +114,9 @@ int femstep_tet_critical_dt(femstep_tet *solver, double youngs, double poisson, 
    writes the mean milliseconds of [0] the element kernel and [1] the node kernel.
    The same arithmetic as femstep_tet_run; used by the benchmark's roofline. */
 int femstep_tet_profile(femstep_tet *solver, int steps, const femstep_tet_params *params, double out[2]);
-/* Number of kernel launches the last femstep_tet_run issued. */
+/* Number of kernel launches the last femstep_tet_run issued: two a step, or one per 1,024
+   steps in a run of 128 steps or more of a mesh small enough for one cluster of blocks (up to
+   8,192 tets and nodes, 4,096 in J2_F64). */
 long long femstep_tet_launches(const femstep_tet *solver);
 const char *femstep_tet_error(const femstep_tet *solver);
 void femstep_tet_destroy(femstep_tet *solver);

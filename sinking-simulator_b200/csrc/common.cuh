@@ -62,9 +62,13 @@ __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch
 // meet at the cluster's hardware barrier twice a step where the two kernels of a step
 // would follow one another, and what no step changes stays in registers.  Forces and
 // displacements go from block to block through L2 (read with __ldcg), ordered by the
-// barrier's release and acquire.  Two kernels a step against one cluster: 960 tets REF32
-// 4.7 -> 3.6 us a step, 4,830 tets FP32 8.8 -> 6.2, 3,840 tets FP64 18.4 -> 17.4 (its polar
-// iteration is the step).  Above 8,192 tets sixteen SMs have more work than the launches cost.
+// barrier's release and acquire.  Two kernels a step against one cluster, us a step: REF32
+// 960 tets 4.8 -> 3.0, 4,830 tets 5.1 -> 4.6, 8,160 tets 5.2 -> 5.0; FP32-K 960 tets
+// 6.2 -> 3.8, 4,830 tets 6.4 -> 4.9, 8,160 tets 6.6 -> 5.7.  8,192 is sixteen blocks of the 512
+// threads that the element's registers allow, where the two meet.  FP64 to 2,048 tets, one
+// group of 128 an SM: 16.0 -> 12.0; from there to 4,096 (kCluster64Most, two groups, which
+// take turns at the FP64 pipe) the two are within 4 %: 2,448 tets 16.4 -> 16.9 us a step,
+// 3,840 tets 17.1 -> 17.1, and a fresh solver's first 400 steps 17.6 -> 16.9.
 constexpr int kClusterBlocks = 16, kClusterMost = 8192;
 constexpr int kClusterSmem = 96 * 1024;  // the most dynamic shared memory a block of one may ask for
 
@@ -128,8 +132,6 @@ __device__ __forceinline__ double block_sum(double v, double* scratch /* >= 32 *
     return total;  // valid in thread 0 only
 }
 
-// Two deterministic block sums in one pass (one pair of barriers): the same order as
-// block_sum for each.  scratch >= 64 doubles.
 // The warp part of block_sum2: each of a and b summed over the warp into lane 0.
 __device__ __forceinline__ void warp_sum2(double& a, double& b) {
     // a warp whose `a` values are all zero (no tet yielded) has the sum zero already
@@ -139,6 +141,8 @@ __device__ __forceinline__ void warp_sum2(double& a, double& b) {
     for (int o = 16; o > 0; o >>= 1) b += __shfl_down_sync(0xffffffffu, b, o);
 }
 
+// Two deterministic block sums in one pass (one pair of barriers): the same order as
+// block_sum for each.  scratch >= 64 doubles.
 __device__ __forceinline__ void block_sum2(double& a, double& b, double* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     warp_sum2(a, b);
@@ -179,8 +183,8 @@ __device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wai
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Running sums of a cluster run's 128-thread groups, each the sums block_sum2 would give a
-// block of 128: put() leaves the warps' sums, and after a barrier add() has the group's
-// first thread add them up in warp order.
+// block of 128: put() leaves the warps' sums, and after a barrier get() gives the sum
+// of the thread's group, added up in warp order.
 struct GroupSums {
     double2 warp[32];
     __device__ __forceinline__ void put(double a, double b) {

@@ -292,8 +292,9 @@ __device__ __forceinline__ void tiled_fill(const PoolDevice& d, const TiledInfo&
 // barriers a tile: one that ends the wait for the gather (and the last tile's node sums,
 // whose stage is then refilled), one between the corner forces and the node sums.  The
 // tile's energy sums are left per warp and added up after the next barrier.  The pass is
-// bound by latency and the L1 pipe together (issue 62 %, L1 72 % busy, 8 blocks of 64
-// registers an SM; 6, 7 and 9 blocks: 516, 494 and 500 us for 458).  256 meshes, 10.99 M
+// bound by latency, issue and the L1 and shared-memory pipe together (each of the two 65 %
+// busy on 982,014 tets, 8 blocks of 64 registers an SM; 6, 7 and 9 blocks: 516, 494 and 500 us
+// for 458).  256 meshes, 10.99 M
 // tets: 491 us with the record, ids and rows read where they were used and four barriers,
 // 458 us so; 128 threads, each with its tet's 18 values, are more warps than two tets a
 // thread would leave.

@@ -527,17 +527,20 @@ __device__ __forceinline__ bool shell_row(const float4* row, float (&j0)[9], flo
     return formed;
 }
 
-// Blocks per SM the register budget is sized for, chosen per launch.  With the
-// operators formed in the kernel the element pass is issue- and latency-bound.  A zone
-// that fills the GPU wants warps to hide latency, more than it minds spills: on the
-// 2 M-element panel 4 blocks (128 registers, 16 warps per SM, ~30 bytes of spill)
-// take 2.49 ms per pass, 5 (96 registers, 20 warps, ~310 bytes of spill to L1)
-// 2.34 ms, 6 (85 registers, ~650 bytes) 2.74 ms.  A zone that fits in one wave is
-// bound by one warp's dependent chain, where every spill reload is latency: on the
-// reference's 2,048-element probe zone 3 blocks (168 registers, no spill) take 18.2 us
-// per step, 4 blocks 19.7 us, 5 blocks 24.0 us.  (All measured before the wide form's
-// state, frames and factor waited in shared memory: at 5 blocks, 130 bytes of spill, the
-// panel's pass takes 1.27 ms now.)
+// Blocks per SM the register budget is sized for, chosen per launch.  A zone of one wave is
+// bound by one warp's dependent chain: the narrow form, 3 blocks (168 registers, no spill),
+// forms each value where it is used.  A zone that fills the GPU wants warps to hide latency:
+// the wide form, 5 blocks (96 registers, some 130 bytes of spill), keeps its state, frames and
+// factor in shared memory (1.27 ms for the 2 M-element panel's pass).  The line is the narrow
+// form's one wave, 7,104 elements.  Both forms, us a step, elastic / 97 % yielded, linear law /
+// the same, Swift:
+//    2,000 elements: narrow 9.3 / 29.3 / 48.0, wide 10.0 / 32.8 / 55.1
+//    7,104:                11.0 / 36.3 / 55.5,      11.3 / 37.4 / 60.1
+//    8,000:                15.5 / 44.4 / 67.9,      12.1 / 39.4 / 62.8
+//   10,000:                16.3 / 39.7 / 62.2,      13.2 / 40.8 / 65.2
+//   15,000:                21.5 / 44.5 / 69.6,      18.7 / 41.3 / 68.6
+// Before the wide form's values waited in shared memory, the panel's pass took 2.49 ms at 4
+// blocks (128 registers), 2.34 at 5 and 2.74 at 6 (85).
 constexpr int kShellMinbWide = 5;
 constexpr int kShellMinbNarrow = 3;
 constexpr int kShellWarpsNarrow = kShellMinbNarrow * kShellBlock / 32;  // per SM
@@ -1267,8 +1270,10 @@ __global__ void __launch_bounds__(kShellBlock, MINB) shell_forces(ShellDevice d,
 // iterations of an element change little from step to step, so the order is renewed once
 // a graph of steps, by one block beside the node pass's.  The results do not depend on it.
 // A yielding bay, step: 35.4 -> 32.5 us with 3 % of its elements yielded, 79.9 -> 71.8 with
-// 81 %; elastic 27.5 -> 27.9 (the lookup).  One wave has no order, and past kShellOrderMost
-// groups (five waves and more) the tail is a small part of the pass.
+// 81 %; elastic 27.5 -> 27.9 (the lookup).  One wave has no order.  The line, kShellOrderMost,
+// is where the slow warps' tail no longer outweighs the lookup and the scattered reads: 65,280
+// elements (16,320 groups) 52.4 -> 53.0 elastic and 61.4 -> 59.7 with 2 % yielded, 89,600
+// 73.9 -> 74.4 and 78.9 -> 79.7, 240,000 192 -> 194 and 203 -> 210.
 // A stable counting sort in four classes, `n` < 2^16, by the block's threads.
 __device__ __noinline__ void shell_order(const uint8_t* cost, uint16_t* order, int* ordered, int n) {
     __shared__ unsigned long long warp_total[kShellNodeBlock / 32];

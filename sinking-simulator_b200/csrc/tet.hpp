@@ -32,8 +32,9 @@
 // would more than double its slots keeps each run contiguous instead).  Contiguous runs
 // made every load of the node pass 32 lines: 19.5 us for the 491,520-tet REF32 mesh
 // (step 39.7 us, L1 72 % busy), with the strided ones the step takes 18.9 us; the
-// 480,000-tet beam 35.6 -> 29.0 us (FP32), 113 -> 94.6 us (FP64); 960 tets 8.3 -> 5.8 us.  No float atomics anywhere; the result does not depend on
-// scheduling.
+// 480,000-tet beam 35.6 -> 29.0 us (FP32), 113 -> 94.6 us (FP64); 960 tets 8.3 -> 5.8 us.
+// No force goes through an atomic, and each slot of the energy account has one writer a
+// launch (account_add): the result does not depend on scheduling.
 #pragma once
 
 #include <cuda_runtime.h>
