@@ -143,6 +143,10 @@ ShellParams make_params(const femstep_shell_params& p) {
     return q;
 }
 
+// Waits for what a call has copied up or cleared on the legacy stream: such a copy from pageable
+// memory may return before it has landed, and the solver's stream does not wait for that stream.
+int settled(femstep_shell* s, const char* what) { return check(s, cudaStreamSynchronize(cudaStreamLegacy), what); }
+
 constexpr int kGraphSteps = 16;
 
 // The readback of a large zone, in slices: each worker copies a slice into its own pinned
@@ -478,6 +482,12 @@ int femstep_shell_create(const femstep_shell_mesh* mesh, femstep_shell** out) {
         a.elem = elem;
         a.corner_mass = corner_mass;
         a.gauss_volume = weights;
+        rc = settled(s, "upload");
+        if (rc) {
+            if (weights) fs::device_free(weights);
+            femstep_shell_destroy(s);
+            return rc;
+        }
         fs::launch_shell_setup(a, s->stream);
         if (corner_mass) fs::launch_shell_mass((long long)N, d.offset, corner_mass, nullptr, mass, inv_mass, s->stream);
         cudaStreamSynchronize(s->stream);
@@ -713,6 +723,7 @@ int femstep_shell_set_punch(femstep_shell* s, const uint32_t* driven, size_t cou
     if (!rc && mass > 0.0 && !list.empty())
         rc = check(s, cudaMemcpy(s->driven_list, list.data(), list.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
                    "punch upload");
+    if (!rc) rc = settled(s, "punch upload");
     if (rc) return rc;
     s->punch = count > 0;
     s->punch_mass = s->punch ? mass : 0.0;
@@ -809,6 +820,7 @@ int femstep_shell_set_edge(femstep_shell* s, const double* prescribed, const dou
                        "edge upload");
         if (!rc) rc = check(s, cudaMemset(s->n_edge, 0, s->nblocks * sizeof(double)), "edge upload");
     }
+    if (!rc) rc = settled(s, "edge upload");
     if (rc) return rc;
     s->d.edge_map = rows > 0 ? s->edge_map : nullptr;
     s->d.edge_base = rows > 0 ? s->edge_rows : nullptr;
@@ -915,6 +927,7 @@ int femstep_shell_set_fibers(femstep_shell* s, const femstep_shell_fibers* f) {
             put(d.inv_mass, im.data(), N * sizeof(float));
         }
     }
+    if (!rc) rc = settled(s, "fibre upload");
     if (rc) return rc;
     d.fibers = (long long)F;
     s->fblocks = fblocks;
@@ -1229,6 +1242,8 @@ int femstep_shell_restore(femstep_shell* s, const void* buffer, size_t bytes) {
         if (rc) return rc;
         in += g.bytes;
     }
+    rc = settled(s, "restore");
+    if (rc) return rc;
     s->punch_time = h.punch_time;
     s->punch_penetration = h.punch_penetration;
     s->punch_steps = h.punch_steps;

@@ -172,3 +172,20 @@ def test_shell_create_makes_few_calls(fake):
         calls.append(fake.lib.fake_calls())
         s.close()
     assert calls[0] == calls[1]
+
+
+def test_shell_settings_land_before_the_next_run(fake):
+    """A punch, a driven edge, fibres and a restored state go up by copies that may return before
+    they have landed; the next run's stream does not wait for them, so the calls do."""
+    s = shell_zone(fake, 6, 5)
+    saved = s.checkpoint()
+    prescribed = np.zeros(3 * s.nodes)
+    prescribed[:3] = 1e-4
+    for setting in (lambda: s.restore(saved), lambda: s.set_punch([1, 3], [0.0, 0.0, -1.0], 1.0),
+                    lambda: s.set_punch([1, 3], [0.0, 0.0, -1.0], 1.0, mass=10.0), lambda: s.set_edge(prescribed),
+                    lambda: s.set_fibers([[0, 1, 12, 13]], [[0.5, 0.5]], [1e-4], density=7850.0)):
+        setting()
+        assert fake.lib.fake_pending() == 0
+        s.run(3, dt=1e-7)
+        assert fake.lib.fake_unordered() == 0
+    s.close()
