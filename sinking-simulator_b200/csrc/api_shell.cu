@@ -452,6 +452,9 @@ int femstep_shell_create(const femstep_shell_mesh* mesh, femstep_shell** out) {
         });
         d.load = A.upload(load.data(), N * 3);
     }
+    // (an allocation waits for the legacy stream: with these two all before them has landed when
+    // the set-up kernels start on the solver's)
+    double* corner_mass = m.mass ? nullptr : A.zeros<double>(E * 8);
     float* mass = A.alloc<float>(N);
     float* inv_mass = A.alloc<float>(N);
     d.mass = mass;
@@ -463,10 +466,8 @@ int femstep_shell_create(const femstep_shell_mesh* mesh, femstep_shell** out) {
     // them for its shaders) must be the solid-shell forms of the same rest positions:
     // every element's Gauss weights, and the whole forms of the first elements, are
     // checked against the device's own FP64 forms.
-    double* corner_mass = nullptr;
     double* weights = nullptr;
     if (A.ok()) {
-        corner_mass = m.mass ? nullptr : A.zeros<double>(E * 8);
         if (m.forms && fs::device_alloc((void**)&weights, E * 8 * sizeof(double)) != cudaSuccess) {
             femstep_shell_destroy(s);
             return fail(nullptr, FEMSTEP_ENOMEM, "device allocation failed");
@@ -482,12 +483,6 @@ int femstep_shell_create(const femstep_shell_mesh* mesh, femstep_shell** out) {
         a.elem = elem;
         a.corner_mass = corner_mass;
         a.gauss_volume = weights;
-        rc = settled(s, "upload");
-        if (rc) {
-            if (weights) fs::device_free(weights);
-            femstep_shell_destroy(s);
-            return rc;
-        }
         fs::launch_shell_setup(a, s->stream);
         if (corner_mass) fs::launch_shell_mass((long long)N, d.offset, corner_mass, nullptr, mass, inv_mass, s->stream);
         cudaStreamSynchronize(s->stream);
